@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
+#include <atomic>
 #include <string>
 #include <vector>
 
@@ -20,6 +21,15 @@ struct NvtxScope {
 #include "common.cuh"
 #include "host_setup.h"
 #include "kernels.cuh"
+
+// A number no other matrix or preconditioner state of the process has had.
+// Captured graphs are looked up by it and not by the object's address, which
+// a later object may get again with other device buffers behind it.
+inline unsigned long long object_uid()
+{
+    static std::atomic<unsigned long long> next{1};
+    return next.fetch_add(1, std::memory_order_relaxed);
+}
 
 struct GraphEntry {
     std::vector<const void *> key;
@@ -51,6 +61,7 @@ struct b200la_ctx {
 };
 
 struct b200la_csr {
+    unsigned long long uid = object_uid();   // renewed whenever a device buffer of the matrix may change
     int n = 0, m = 0, nnz = 0, dtype = 0, lg = 0, cfg = 0;
     int *row = nullptr, *col = nullptr;
     void *val = nullptr;
@@ -98,6 +109,7 @@ struct b200la_csr {
 };
 
 struct b200la_precond {
+    unsigned long long uid = object_uid();
     int kind = 0, n = 0, dtype = 0;
     void *invd = nullptr;             // Jacobi: 1/a_ii
     // block sweeps (colours / levels) in the permuted numbering

@@ -762,6 +762,7 @@ extern "C" int b200la_csr_cast(b200la_ctx *ctx, const b200la_csr *A, int dtype, 
 {
     if (!ctx || !A || !out || (dtype != B200LA_F64 && dtype != B200LA_F32)) return B200LA_ERR_ARG;
     b200la_csr *B = new b200la_csr(*A);
+    B->uid = object_uid();
     B->dtype = dtype;
     B->row = nullptr;
     B->col = nullptr;
@@ -877,6 +878,7 @@ extern "C" int b200la_csr_set_values(b200la_ctx *ctx, b200la_csr *A, const void 
     if (A->nnz) CK(cudaMemcpyAsync(A->val, val, dsize(A->dtype) * A->nnz, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     drop_invd32(A);
+    A->uid = object_uid();
     int rc = build_sell(ctx, A);
     if (!rc) rc = build_stencil(ctx, A);
     return rc ? rc : lattice_refresh(ctx, A);
@@ -889,6 +891,7 @@ extern "C" int b200la_csr_scale(b200la_ctx *ctx, b200la_csr *A, double alpha, in
     if (A->nnz) CK(launch_csr_scale(A->dtype, A->n, A->row, A->col, A->val, alpha, mode, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     drop_invd32(A);
+    A->uid = object_uid();
     // the SpMV layouts derived from the values follow them
     int rc = build_sell(ctx, A);
     if (!rc) rc = build_stencil(ctx, A);

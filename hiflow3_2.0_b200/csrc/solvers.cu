@@ -40,6 +40,16 @@ static int batch_size()
     return 16;
 }
 
+// The parts of a graph's key that stand for the objects whose buffers it
+// holds: their numbers, and for a Jacobi preconditioner (which may be a
+// temporary) its one buffer.
+static const void *graph_key(const b200la_csr *A) { return reinterpret_cast<const void *>((uintptr_t)A->uid); }
+static const void *graph_key(const b200la_precond *P)
+{
+    if (!P || P->kind == B200LA_PRECOND_JACOBI) return P ? P->invd : nullptr;
+    return reinterpret_cast<const void *>((uintptr_t)P->uid);
+}
+
 // Capture `body` (which enqueues kernels on ctx->stream) into a graph keyed by
 // `key`, or reuse the cached one.  Returns the executable graph.
 template <class Body>
@@ -236,7 +246,7 @@ static int cg_core(b200la_ctx *ctx, const b200la_csr *A, const b200la_precond *P
         }
     }
     const bool loop = !no_graph && loop_policy();
-    const std::vector<const void *> key = {A, P, b, x, w.r, w.p, w.Ap, w.z, (const void *)(intptr_t)K,
+    const std::vector<const void *> key = {graph_key(A), graph_key(P), b, x, w.r, w.p, w.Ap, w.z, (const void *)(intptr_t)K,
                                            (const void *)(intptr_t)pc, ctx->stream, (const void *)(intptr_t)loop};
     auto batch = [&]() -> int {
         for (int k = 0; k < K; ++k) {
@@ -727,8 +737,9 @@ extern "C" int b200la_gmres(b200la_ctx *ctx, const b200la_csr *A, const b200la_p
         };
         cudaGraphExec_t exec;
         int nodes = 0;
-        rc = get_graph(ctx, {A, P, b, x, wk, (const void *)(intptr_t)mb, (const void *)(intptr_t)(-7), ctx->stream},
-                       cycle, &exec, &nodes);
+        const int kind = P ? P->kind : 0;
+        rc = get_graph(ctx, {graph_key(A), graph_key(P), b, x, wk, (const void *)(intptr_t)mb,
+                             (const void *)(intptr_t)(-7 - kind), ctx->stream}, cycle, &exec, &nodes);
         if (rc) return rc;
         SK(cudaGraphLaunch(exec, ctx->stream));
         graph_launches += nodes;

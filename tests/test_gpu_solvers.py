@@ -340,6 +340,46 @@ def test_ilu0_level_sweep_beyond_ring(pf, b200, dim, N, kind, monkeypatch):
 
 
 
+def test_captured_graphs_follow_new_objects(pf, b200):
+    """A solve after its operator and preconditioner were freed and others made
+    (whose handles may get the freed addresses again) runs on the new ones: the
+    captured iterations are found by the objects, not by their addresses."""
+    import scipy.sparse as sp
+    import scipy.sparse.linalg as sl
+    N = 16
+    n = (N + 1) ** 2
+    b, x = pf.vector(n), pf.vector(n)
+    for k in range(5):
+        row, col, val = b200.q1_assemble(2, N, 1, None, 0.05 * (k + 1), (1.0, 0.5))
+        bh = b200.q1_rhs(42 + k, 2, N)
+        P = b200.Preconditioner.ILU0(pf, row, col, val, b200.PRECOND_ILU0_LS if k % 2 else b200.PRECOND_ILU0_MC)
+        b.CopyFrom(pf.vector(bh[P.perm]))
+        gm = b200.GMRES(pf, 30)
+        gm.SetupOperator(P.A_perm)
+        gm.SetupPreconditioner(P)
+        gm.InitControl(1000, 0.0, 1e-10, 1e6)
+        x.Zeros()
+        assert gm.Solve(b, x) == b200.SUCCESS_REL
+        ref = sl.spsolve(sp.csc_matrix(sp.csr_matrix((val, col, row), shape=(n, n))), bh)[P.perm]
+        assert np.linalg.norm(x.numpy() - ref) <= 1e-8 * np.linalg.norm(ref)
+        row, col, val = b200.q1_assemble(2, N, 0, np.full(N * N, k + 1.0))
+        A = b200.CSR_lMatrix.from_csr(pf, row, col, val)
+        cg = b200.CG(pf)
+        cg.SetupOperator(A)
+        cg.SetupPreconditioner(b200.Preconditioner.Jacobi(pf, A))
+        cg.InitControl(1000, 0.0, 1e-10, 1e6)
+        for scale in (1.0, 2.0):          # the same object with other values
+            if scale != 1.0:
+                A.Scale(scale)
+                cg.SetupPreconditioner(b200.Preconditioner.Jacobi(pf, A))
+            b.CopyFrom(pf.vector(bh))
+            x.Zeros()
+            assert cg.Solve(b, x) == b200.SUCCESS_REL
+            ref = sl.spsolve(sp.csc_matrix(sp.csr_matrix((val * scale, col, row), shape=(n, n))), bh)
+            assert np.linalg.norm(x.numpy() - ref) <= 1e-8 * np.linalg.norm(ref)
+        del P, A, gm, cg
+
+
 @pytest.mark.parametrize("precond", ["none", "jacobi", "mcsgs"])
 def test_device_loop_matches_host_batches(pf, b200, monkeypatch, precond):
     """The CG iterations run in a device-side while loop (one graph launch per
