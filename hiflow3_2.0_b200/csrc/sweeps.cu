@@ -16,9 +16,11 @@
 #include "b200la_internal.h"
 
 #include <algorithm>
+#include <climits>
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 using namespace b200;
@@ -274,161 +276,382 @@ __global__ void __launch_bounds__(kLevelThreads) level_sweep_cta_kernel(LevelSwe
     }
 }
 
-// The level sweep with a deeper look-ahead through the async-copy engine.
-// At set-up every row of L / U is packed into kp fixed slots (columns and
-// values, the entry count beside).  Each thread copies its row of level
-// k + kStages - 1 (packed entries, count, own input and scalings) into a
-// shared-memory stage with cp.async while level k is solved, so the loads of
-// a level arrive kStages - 1 levels early and only the ring gathers, the
-// solve and the level barrier remain on the critical path.
-constexpr int kStages = 4;
-constexpr int kRingStaged = 4096;
-constexpr int kStagedMaxLevels = 4096;
-constexpr int kStagedSlots = 4;    // packed entries per row (rows of L and U with at most this many)
+// The level sweep on a packed stream of the factor, both directions in one
+// launch.  At set-up the rows of L and U are packed, in dependency order, into
+// tiles of at most pack_rows(KP) consecutive rows of one level: a 16-byte
+// header (first row, rows) and one record per row -- the values, where their
+// vector entries lie (16-bit byte offsets) and the diagonal scalings.
+// Producer warps bring each tile and the rows' own inputs (r, then the forward
+// result) into a ring of shared-memory stages by bulk copies, several tiles
+// ahead; the other warps solve one row per thread.  The results of the last
+// kPackRing rows stay in shared memory, where the next levels gather them;
+// entries further back (the identity rows of level 0, for instance) are copied
+// ahead by the producer into slots of the stage.
+//   The sweep is a serial chain of levels: what bounds it is the instruction
+// stream of one level, not its bytes (about 60 per FP64 row of four entries).
+// So a level's records are read while the level before it is solved, its
+// header a level earlier still, a watching warp does the waiting for tiles, and
+// between two barriers stand one gather per entry, the products in column order
+// and the store into the ring.  Four producer warps: one needs about 1,000
+// cycles per tile.  One CTA: across SMs every level would wait for a cluster
+// barrier and for remote shared memory.
+//   Measured (one apply, both directions; before: one cp.async look-ahead per
+// thread for rows of up to four entries, a register look-ahead for longer
+// ones): 2-D 512^2 ILU(0), 1,537 levels, FP64 2,470 -> 695 us (0.23 us per
+// level); 256^2 1,060 -> 292 us, FP32 230 us; 150^2 ILU(1) 1,880 -> 390 us.
+constexpr int kPackMaxRows = 512;
+constexpr int pack_rows(int kp) { return kp == 4 ? kPackMaxRows : kp == 8 ? 256 : 192; }   // rows of a tile
+constexpr int kPackMaxStages = 8;
+constexpr int kPackMinStages = 4;
+constexpr int kPackRing = 4096;    // at least kPackMaxStages tiles, so that what lies further back is solved
+constexpr int kPackProducers = 4;   // producer warps
+constexpr int kPackFar = 32;       // far entries of a tile
+constexpr int kPackMaxEntries = 16;
+constexpr size_t kPackSmemCap = 225 * 1024;   // of the 227 KB a CTA can have, less the static part
+static_assert(kPackRing >= kPackMaxStages * kPackMaxRows, "far entries must be solved when their tile is issued");
 
-struct LevelStagedArgs {
-    const int *pcol;      // packed columns [n][kp]
-    const void *pval;     // packed values [n][kp]
-    const int *pcnt;      // entries per row
-    const int *off;
-    int nlev, n;
+struct alignas(16) PackTile {
+    int row0, m;
+    unsigned off16;          // the tile's packed bytes start at 16 * off16
+    int far0, nfar;          // its far columns
+    int pad[3];
+};
+
+struct PackedSweepArgs {
+    const PackTile *tiles;          // forward tiles, then backward tiles
+    const unsigned char *pack;
+    const int *far;                 // far columns of all tiles, and their number
+    int nf, nt;                     // forward tiles, all tiles
+    int nfar, n, stages, stage_bytes, own_off;
     const void *r;
     void *z;
-    const void *d1, *d2;
-    int backward, sgs;
     const int *gate;
+    int *err;
 };
 
-__device__ __forceinline__ void cp_async(void *dst, const void *src, int bytes)
+// Row record: KP values, KP offsets, one scaling (two for SGS); padded so that
+// the eight lanes of a 16-byte shared-memory phase fall on different banks.
+template <typename T, int KP, bool SGS>
+struct PackRec {
+    static constexpr int scal = KP * (int)sizeof(T) + 2 * KP;
+    static constexpr int used = (scal + (SGS ? 2 : 1) * (int)sizeof(T) + 15) & ~15;
+    static constexpr int bytes = (used / 16) % 2 == 1 ? used : used + 16;
+};
+// shared memory before the stages: the ring, a zero entry, the stages' far entries
+template <typename T>
+__host__ __device__ constexpr int pack_far_off() { return kPackRing * (int)sizeof(T) + 16; }
+template <typename T>
+__host__ __device__ constexpr int pack_head_bytes()
 {
-    const unsigned d = smem_u32(dst);
-    if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-    else if (bytes == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+    return pack_far_off<T>() + kPackMaxStages * kPackFar * (int)sizeof(T);
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+static_assert(pack_head_bytes<double>() <= 65536, "16-bit offsets");
 
-template <typename T, int KP>
-struct StageRec {
-    int col[KP];
-    T val[KP];
-    T own, e1, e2;
-    int cnt;
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// arrives when the calling thread's cp.async copies so far have landed
+__device__ __forceinline__ void mbar_arrive_cp_async(uint64_t *bar)
+{
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+template <typename T>
+__device__ __forceinline__ void cp_async_one(void *dst, const T *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(sizeof(T)) : "memory");
+}
+
+struct PackedShared {
+    uint64_t full[kPackMaxStages], empty[kPackMaxStages], fwd_done;
+    int fail;
 };
 
-template <typename T, int KP>
-__global__ void __launch_bounds__(kLevelThreads) level_sweep_staged_kernel(LevelStagedArgs a)
+// The barrier between two tiles, of the solving warps and the watching warp.
+__device__ __forceinline__ void packed_barrier(int threads)
 {
-    // one thread per row of the largest level (blockDim.x <= kLevelThreads):
-    // idle warps would only lengthen every level's barrier
-    const int NT = blockDim.x;
-    extern __shared__ __align__(16) unsigned char s_raw[];
-    using Rec = StageRec<T, KP>;
-    Rec *stage = reinterpret_cast<Rec *>(s_raw);                             // [kStages][NT]
-    T *ring = reinterpret_cast<T *>(s_raw + sizeof(Rec) * kStages * NT);
-    int *s_off = reinterpret_cast<int *>(ring + kRingStaged);
-    if (gate_closed(a.gate)) return;
-    for (int i = threadIdx.x; i <= a.nlev; i += NT) s_off[i] = __ldg(a.off + i);
-    __syncthreads();
-    const int tid = threadIdx.x, nlev = a.nlev;
-    const T *pval = static_cast<const T *>(a.pval);
-    const T *r = static_cast<const T *>(a.r);
-    const T *d1 = static_cast<const T *>(a.d1);
-    const T *d2 = static_cast<const T *>(a.d2);
+    asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+}
+
+template <typename T, int KP>
+struct PackedRow {
+    T v[KP];
+    unsigned ix[KP / 2];   // byte offsets of the row's vector entries, in pairs
+    int at[KP];            // and unpacked
+    T own, e1, e2;
+};
+
+// One direction of the sweep, by the solving threads: cnt tiles, the first of
+// them in stage `stg`.  A tile may be read from the barrier before the tile
+// ahead of it on (the watching warp has seen it arrive).
+template <typename T, int KP, bool SGS, bool BWD>
+__device__ __forceinline__ void packed_phase(const PackedSweepArgs &a, unsigned char *smem, int cnt, int &stg, int NT)
+{
+    using Rec = PackRec<T, KP, SGS>;
+    constexpr int R = Rec::bytes;
+    const int tid = threadIdx.x, S = a.stages;
     T *z = static_cast<T *>(a.z);
-    const bool need_e1 = a.backward || a.sgs, need_e2 = a.backward && a.sgs;
-    auto level_of = [&](int k) { return a.backward ? nlev - 1 - k : k; };
-    // this thread's row of level k into stage k % kStages (one commit group per level)
-    auto issue = [&](int k) {
-        if (k < nlev) {
-            const int l = level_of(k), rr = s_off[l] + tid;
-            if (rr < s_off[l + 1]) {
-                Rec &q = stage[(k % kStages) * NT + tid];
+    const T *vec = BWD ? z : static_cast<const T *>(a.r);
+    constexpr unsigned W = 16 / sizeof(T) - 1;
+    const unsigned vsh = (unsigned)(reinterpret_cast<uintptr_t>(vec) / sizeof(T)) & W;   // first element in its 16 bytes
+    const unsigned char *stages = smem + pack_head_bytes<T>();
+    const unsigned char *rec_at = stages + 16 + tid * R;
+    const T *own_at = reinterpret_cast<const T *>(stages + a.own_off) + tid;
+    auto next = [&](int s) { return s + 1 == S ? 0 : s + 1; };
+    auto header = [&](int s) { return *reinterpret_cast<const int2 *>(stages + s * a.stage_bytes); };
+    auto record = [&](PackedRow<T, KP> &q, int s, int2 h) {
+        if (tid >= h.y) return;
+        const uint4 *p = reinterpret_cast<const uint4 *>(rec_at + s * a.stage_bytes);
+        uint4 w[Rec::used / 16];
 #pragma unroll
-                for (int b = 0; b < KP * 4; b += 16) cp_async(reinterpret_cast<char *>(q.col) + b,
-                                                              reinterpret_cast<const char *>(a.pcol + (size_t)rr * KP) + b, 16);
+        for (int i = 0; i < Rec::used / 16; ++i) w[i] = p[i];
+        const unsigned *u = reinterpret_cast<const unsigned *>(w);
+        auto get = [&](int byte) -> T {
+            if constexpr (sizeof(T) == 8) return __hiloint2double((int)u[byte / 4 + 1], (int)u[byte / 4]);
+            else return __uint_as_float(u[byte / 4]);
+        };
 #pragma unroll
-                for (int b = 0; b < KP * (int)sizeof(T); b += 16)
-                    cp_async(reinterpret_cast<char *>(q.val) + b, reinterpret_cast<const char *>(pval + (size_t)rr * KP) + b,
-                             16);
-                cp_async(&q.cnt, a.pcnt + rr, 4);
-                cp_async(&q.own, (a.backward ? static_cast<const T *>(z) : r) + rr, (int)sizeof(T));
-                if (need_e1) cp_async(&q.e1, d1 + rr, (int)sizeof(T));
-                if (need_e2) cp_async(&q.e2, d2 + rr, (int)sizeof(T));
-            }
-        }
-        cp_async_commit();
+        for (int e = 0; e < KP; ++e) q.v[e] = get(e * (int)sizeof(T));
+#pragma unroll
+        for (int e = 0; e < KP / 2; ++e) q.ix[e] = u[KP * (int)sizeof(T) / 4 + e];
+        if (BWD || SGS) q.e1 = get(Rec::scal);
+        if (BWD && SGS) q.e2 = get(Rec::scal + (int)sizeof(T));
+        q.own = reinterpret_cast<const T *>(reinterpret_cast<const unsigned char *>(own_at) +
+                                            s * a.stage_bytes)[(vsh + (unsigned)h.x) & W];
     };
-    auto solve = [&](int rr, const int *cols, const T *vals, int cnt, T own, T e1, T e2, int r0, int r1) {
+    // (apart from the loads: it waits for them)
+    auto unpack = [&](PackedRow<T, KP> &q) {
+#pragma unroll
+        for (int e = 0; e < KP; ++e) q.at[e] = (int)(e & 1 ? q.ix[e / 2] >> 16 : q.ix[e / 2] & 0xffffu);
+    };
+    int s1 = next(stg), s2 = next(s1);
+    packed_barrier(NT + 32);   // the first two tiles are there
+    int2 hc = header(stg), hn = cnt > 1 ? header(s1) : make_int2(0, 0);
+    PackedRow<T, KP> ra, rb;
+    record(ra, stg, hc);
+    unpack(ra);
+    auto step = [&](PackedRow<T, KP> &cur, PackedRow<T, KP> &nxt, int k) {
+        const bool active = tid < hc.y;
+        T g[KP];
+#pragma unroll
+        for (int e = 0; e < KP; ++e) g[e] = active ? *reinterpret_cast<const T *>(smem + cur.at[e]) : T(0);
+        record(nxt, s1, hn);
         T s = T(0);
 #pragma unroll
-        for (int e = 0; e < KP; ++e) {
-            if (e < cnt) {
-                const int cc = cols[e];
-                const bool in_ring = a.backward ? cc < r0 + kRingStaged : cc >= r1 - kRingStaged;
-                s += vals[e] * (in_ring ? ring[cc & (kRingStaged - 1)] : __ldcg(z + cc));
-            }
-        }
+        for (int e = 0; e < KP; ++e) s += cur.v[e] * g[e];
         T out;
-        if (!a.backward) out = a.sgs ? (-own + s) * e1 : -(-own + s);
-        else out = a.sgs ? (own * e2 + s) * e1 : (-own + s) * e1;
-        ring[rr & (kRingStaged - 1)] = out;
-        __stcg(z + rr, out);
+        if (!BWD) out = SGS ? (-cur.own + s) * cur.e1 : -(-cur.own + s);
+        else out = SGS ? (cur.own * cur.e2 + s) * cur.e1 : (-cur.own + s) * cur.e1;
+        if (active) {
+            const int rr = hc.x + tid;
+            reinterpret_cast<T *>(smem)[rr & (kPackRing - 1)] = out;
+            z[rr] = out;
+        }
+        unpack(nxt);
+        if (!BWD && k + 1 == cnt) asm volatile("fence.proxy.async.global;" ::: "memory");   // z before its bulk copies
+        packed_barrier(NT + 32);
+        hc = hn;
+        hn = k + 2 < cnt ? header(s2) : make_int2(0, 0);
+        s1 = s2;
+        s2 = next(s2);
     };
-#pragma unroll
-    for (int k = 0; k < kStages - 1; ++k) issue(k);
-    for (int k = 0; k < nlev; ++k) {
-        issue(k + kStages - 1);
-        cp_async_wait<kStages - 1>();
-        const int l = level_of(k), r0 = s_off[l], r1 = s_off[l + 1];
-        const int rr = r0 + tid;
-        if (rr < r1) {
-            const Rec &q = stage[(k % kStages) * NT + tid];
-            solve(rr, q.col, q.val, q.cnt, q.own, need_e1 ? q.e1 : T(0), need_e2 ? q.e2 : T(0), r0, r1);
-        }
-        // rows of a level beyond the first NT: read directly
-        for (int r2 = rr + NT; r2 < r1; r2 += NT) {
-            int cols[KP];
-            T vals[KP];
-#pragma unroll
-            for (int e = 0; e < KP; ++e) {
-                cols[e] = __ldg(a.pcol + (size_t)r2 * KP + e);
-                vals[e] = __ldg(pval + (size_t)r2 * KP + e);
-            }
-            const T own = a.backward ? __ldcg(z + r2) : r[r2];
-            solve(r2, cols, vals, __ldg(a.pcnt + r2), own, need_e1 ? d1[r2] : T(0), need_e2 ? d2[r2] : T(0), r0, r1);
-        }
-        __syncthreads();
+    for (int k = 0; k < cnt; k += 2) {
+        step(ra, rb, k);
+        if (k + 1 < cnt) step(rb, ra, k + 1);
     }
-    cp_async_wait<0>();
+    stg = (stg + cnt) % S;
 }
 
-// Pack the rows of a CSR into kp fixed slots (columns, values; unused slots
-// column 0, value 0) with the entry count beside.
-template <typename T>
-__global__ void pack_rows_kernel(int n, int kp, const int *__restrict__ row, const int *__restrict__ col,
-                                 const T *__restrict__ val, int *__restrict__ pcol, T *__restrict__ pval,
-                                 int *__restrict__ pcnt)
+template <typename T, int KP, bool SGS>
+__global__ void __launch_bounds__(pack_rows(KP) + 32 * (1 + kPackProducers), 1)
+    level_sweep_packed_kernel(PackedSweepArgs a)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int b = row[i], e = row[i + 1];
-        for (int k = 0; k < kp; ++k) {
-            const bool in = b + k < e;
-            pcol[(size_t)i * kp + k] = in ? col[b + k] : 0;
-            pval[(size_t)i * kp + k] = in ? val[b + k] : T(0);
+    if (gate_closed(a.gate)) return;
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    __shared__ PackedShared sh;
+    const int tid = threadIdx.x, NT = blockDim.x - 32 * (1 + kPackProducers), S = a.stages, nf = a.nf, nt = a.nt;
+    if (tid == 0) {
+        for (int i = 0; i < kPackMaxStages; ++i) {
+            mbar_init(&sh.full[i], a.nfar ? 1 + 32 : 1);
+            mbar_init(&sh.empty[i], 1);
         }
-        pcnt[i] = e - b;
+        mbar_init(&sh.fwd_done, 1);
+        fence_mbar_init();
+        sh.fail = 0;
+        *reinterpret_cast<T *>(s_raw + kPackRing * sizeof(T)) = T(0);
     }
+    __syncthreads();
+    if (tid < NT) {
+        int stg = 0;
+        packed_phase<T, KP, SGS, false>(a, s_raw, nf, stg, NT);
+        packed_phase<T, KP, SGS, true>(a, s_raw, nt - nf, stg, NT);
+        return;
+    }
+    // bounded waits: after one has run out (reported in *err) nothing waits any more
+    auto wait = [&](uint64_t *bar, unsigned parity) {
+        if (mbar_try_wait(bar, parity)) return true;
+        volatile int *fail = &sh.fail;
+        if (!*fail && !mbar_wait_bounded(bar, parity, a.err)) *fail = 1;
+        return *fail == 0;
+    };
+    const int lane = tid & 31, w = ((tid - NT) >> 5) - 1;
+    if (w < 0) {
+        // Watching warp: it meets the barrier after a tile once the tile two
+        // ahead has arrived, and hands the solved tile's stage back, so that
+        // the solving warps look at no arrival barrier themselves.
+        for (int k0 = 0, k1 = nf; k0 < nt; k0 = k1, k1 = nt) {
+            for (int q = k0; q < min(k0 + 2, k1); ++q) wait(&sh.full[q % S], (unsigned)(q / S) & 1u);
+            packed_barrier(NT + 32);
+            int s = k0 % S, s2 = (k0 + 2) % S;
+            unsigned p2 = (unsigned)((k0 + 2) / S) & 1u;
+            for (int k = k0; k < k1; ++k) {
+                if (k + 2 < k1) wait(&sh.full[s2], p2);
+                packed_barrier(NT + 32);
+                if (lane == 0) mbar_arrive(&sh.empty[s]);
+                if (++s == S) s = 0;
+                if (++s2 == S) {
+                    s2 = 0;
+                    p2 ^= 1u;
+                }
+            }
+            if (k1 == nf && lane == 0) mbar_arrive(&sh.fwd_done);
+        }
+        return;
+    }
+    // Producer warps, tile k by warp k % kPackProducers; descriptors and far
+    // columns are read ahead (a load per tile on its own path would put a
+    // memory round trip into every level).
+    const uint64_t pol = l2_policy(0);
+    constexpr int W = 16 / (int)sizeof(T) - 1;
+    T *z = static_cast<T *>(a.z);
+    auto tile_at = [&](int k) { return a.tiles[min(k, nt - 1)]; };
+    auto far_at = [&](const PackTile &t) { return lane < t.nfar ? __ldg(a.far + t.far0 + lane) : 0; };
+    PackTile t = tile_at(w), t1 = tile_at(w + kPackProducers);
+    int f = far_at(t), k = w;
+    bool backward = false;
+    for (; k < nt; k += kPackProducers) {
+        const PackTile t2 = tile_at(k + 2 * kPackProducers);
+        const int f1 = far_at(t1), s = k % S;
+        bool ok = k < S || wait(&sh.empty[s], (unsigned)(k / S - 1) & 1u);
+        if (!backward && k >= nf) {   // the backward inputs are the forward results
+            ok = wait(&sh.fwd_done, 0u) && ok;
+            backward = true;
+        }
+        if (!__all_sync(0xffffffffu, ok)) break;
+        unsigned char *st = s_raw + pack_head_bytes<T>() + (size_t)s * a.stage_bytes;
+        if (lane < t.nfar) cp_async_one(reinterpret_cast<T *>(s_raw + pack_far_off<T>()) + s * kPackFar + lane, z + f);
+        if (lane == 0) {
+            // own inputs: the 16-byte units around [row0, row0 + m); at the
+            // vector's ragged ends the elements inside it one by one
+            const T *vec = backward ? z : static_cast<const T *>(a.r);
+            const int sft = (int)(((unsigned)(reinterpret_cast<uintptr_t>(vec) / sizeof(T)) + (unsigned)t.row0) & W);
+            int q0 = t.row0 - sft, q1 = q0 + ((sft + t.m + W) & ~W);
+            T *own = reinterpret_cast<T *>(st + a.own_off) + sft - t.row0;   // own[i] for row i
+            if (q0 < 0 || q1 > a.n) {
+                if (q0 < 0) q0 += W + 1;
+                if (q1 > a.n) q1 -= W + 1;
+                if (q1 < q0) q0 = q1 = t.row0 + t.m;
+                for (int i = t.row0; i < t.row0 + t.m; ++i)
+                    if (i < q0 || i >= q1) own[i] = __ldcg(vec + i);
+            }
+            const unsigned ob = (unsigned)(q1 - q0) * (unsigned)sizeof(T);
+            const unsigned bytes = 16u + (unsigned)(t.m * PackRec<T, KP, SGS>::bytes);
+            mbar_arrive_expect_tx(&sh.full[s], bytes + ob);
+            bulk_g2s(st, a.pack + 16 * (size_t)t.off16, bytes, &sh.full[s], pol);
+            if (ob) bulk_g2s(own + q0, vec + q0, ob, &sh.full[s], pol);
+        }
+        if (a.nfar) mbar_arrive_cp_async(&sh.full[s]);
+        t = t1;
+        t1 = t2;
+        f = f1;
+    }
+    if (k < nt)   // a wait has run out: leave none of this warp's copies in flight
+        for (int q = w; q < k; q += kPackProducers)
+            if (q >= k - S) mbar_wait_bounded(&sh.full[q % S], (unsigned)(q / S) & 1u, a.err);
 }
 
-constexpr size_t kStagedSmemCap = 226 * 1024;   // opt-in shared memory per CTA on sm_100 (227 KB), less the static part
+// Set-up: the far columns of every tile (fill = 0: counted into nfar[], fill =
+// 1: listed at far0 in row order), and the packed tiles.  One warp per tile.
+__device__ __forceinline__ bool pack_is_far(bool bwd, int r0, int r1, int c)
+{
+    return (bwd ? c - r0 + 1 : r1 - c) > kPackRing;
+}
+__global__ void pack_far_kernel(int nt, int nf, PackTile *tiles, const int *__restrict__ rl, const int *__restrict__ cl,
+                                const int *__restrict__ ru, const int *__restrict__ cu, int fill, int *far)
+{
+    const int k = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
+    if (k >= nt) return;
+    const bool bwd = k >= nf;
+    const int *row = bwd ? ru : rl, *col = bwd ? cu : cl;
+    const int r0 = tiles[k].row0, r1 = r0 + tiles[k].m, far0 = tiles[k].far0, end = row[r1];
+    int c = 0;
+    for (int j0 = row[r0]; j0 < end; j0 += 32) {
+        const int cj = j0 + lane < end ? col[j0 + lane] : 0;
+        const bool is = j0 + lane < end && pack_is_far(bwd, r0, r1, cj);
+        const unsigned b = __ballot_sync(0xffffffffu, is);
+        if (fill && is) far[far0 + c + __popc(b & ((1u << lane) - 1u))] = cj;
+        c += __popc(b);
+    }
+    if (!fill && lane == 0) tiles[k].nfar = c;
+}
+
+template <typename T, int KP, bool SGS>
+__global__ void pack_tiles_kernel(int nt, int nf, const PackTile *__restrict__ tiles, const int *__restrict__ rl,
+                                  const int *__restrict__ cl, const T *__restrict__ vl, const int *__restrict__ ru,
+                                  const int *__restrict__ cu, const T *__restrict__ vu, const T *__restrict__ d1,
+                                  const T *__restrict__ d2, int stages, unsigned char *__restrict__ pack)
+{
+    const int k = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
+    if (k >= nt) return;
+    const bool bwd = k >= nf;
+    const PackTile t = tiles[k];
+    const int *row = bwd ? ru : rl, *col = bwd ? cu : cl;
+    const T *val = bwd ? vu : vl;
+    unsigned char *st = pack + 16 * (size_t)t.off16;
+    if (lane == 0) *reinterpret_cast<int4 *>(st) = make_int4(t.row0, t.m, 0, 0);
+    const int slot0 = pack_far_off<T>() + (k % stages) * kPackFar * (int)sizeof(T);
+    int far_before = 0;   // far entries of the rows of earlier passes
+    for (int i0 = 0; i0 < t.m; i0 += 32) {
+        const int i = i0 + lane, rr = t.row0 + i;
+        const int b = i < t.m ? row[rr] : 0, cnt = i < t.m ? row[rr + 1] - b : 0;
+        int fc = 0;
+        for (int e = 0; e < cnt; ++e) fc += pack_is_far(bwd, t.row0, t.row0 + t.m, col[b + e]);
+        int incl = fc;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        int slot = far_before + incl - fc;
+        far_before += __shfl_sync(0xffffffffu, incl, 31);
+        if (i < t.m) {
+            unsigned char *q = st + 16 + (size_t)i * PackRec<T, KP, SGS>::bytes;
+            T *v = reinterpret_cast<T *>(q);
+            unsigned short *ix = reinterpret_cast<unsigned short *>(q + KP * sizeof(T));
+            for (int e = 0; e < KP; ++e) {
+                v[e] = e < cnt ? val[b + e] : T(0);
+                int off = kPackRing * (int)sizeof(T);   // the zero entry
+                if (e < cnt) {
+                    const int c = col[b + e];
+                    off = pack_is_far(bwd, t.row0, t.row0 + t.m, c) ? slot0 + (slot++) * (int)sizeof(T)
+                                                                    : (c & (kPackRing - 1)) * (int)sizeof(T);
+                }
+                ix[e] = (unsigned short)off;
+            }
+            T *sc = reinterpret_cast<T *>(q + PackRec<T, KP, SGS>::scal);
+            sc[0] = d1[rr];
+            if (SGS) sc[1] = d2[rr];
+        }
+    }
+}
 
 template <typename T, int KP>
-size_t staged_smem(int nlev, int NT = kLevelThreads)
+cudaError_t packed_attr()
 {
-    return sizeof(StageRec<T, KP>) * kStages * NT + sizeof(T) * kRingStaged + sizeof(int) * (nlev + 1);
+    cudaError_t e = cudaFuncSetAttribute(level_sweep_packed_kernel<T, KP, false>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPackSmemCap);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(level_sweep_packed_kernel<T, KP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)kPackSmemCap);
 }
 
 }  // namespace
@@ -438,14 +661,8 @@ namespace b200 {
 cudaError_t sweeps_configure()
 {
     cudaError_t e;
-    // the largest stage set a plan may use (its CTA size and level count are
-    // checked against kStagedSmemCap at set-up)
-    if ((e = cudaFuncSetAttribute(level_sweep_staged_kernel<double, kStagedSlots>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)std::min(staged_smem<double, kStagedSlots>(kStagedMaxLevels), kStagedSmemCap))) ||
-        (e = cudaFuncSetAttribute(level_sweep_staged_kernel<float, kStagedSlots>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)std::min(staged_smem<float, kStagedSlots>(kStagedMaxLevels), kStagedSmemCap))))
+    if ((e = packed_attr<double, 4>()) || (e = packed_attr<double, 8>()) || (e = packed_attr<double, 16>()) ||
+        (e = packed_attr<float, 4>()) || (e = packed_attr<float, 8>()) || (e = packed_attr<float, 16>()))
         return e;
     e = cudaFuncSetAttribute(level_sweep_cta_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)(kLevelRing * sizeof(double) + sizeof(int) * (kLevelMaxLevels + 1)));
@@ -486,11 +703,11 @@ struct SyncFreePlan {
     int lg_l = 0, lg_u = 0;
     int *lev_off = nullptr;   // single-CTA level sweep: level offsets (null: chunk tickets)
     int nlev = 0;
-    // staged variant: rows of L / U packed into kStagedSlots slots
-    int staged = 0;
-    int threads = kLevelThreads;   // the largest level's rows rounded up to a warp (at most kLevelThreads)
-    int *pcol[2] = {nullptr, nullptr}, *pcnt[2] = {nullptr, nullptr};
-    void *pval[2] = {nullptr, nullptr};
+    // packed variant (kp > 0): the tiles and the packed stream of both sweeps
+    int kp = 0, threads = 0, nf_tiles = 0, nt_tiles = 0, stages = 0, stage_bytes = 0, own_off = 0, nfar = 0;
+    PackTile *ptiles = nullptr;
+    int *far = nullptr;
+    unsigned char *pack = nullptr;
 };
 
 static int lanes_for(const b200la_csr *M)
@@ -501,74 +718,136 @@ static int lanes_for(const b200la_csr *M)
     return lg;
 }
 
+// The packed plan of P's sweeps; plan->kp stays 0 when the operator does not
+// fit it (rows too long, too many far columns in a tile).
+template <typename T, int KP, bool SGS>
+static cudaError_t packed_setup(b200la_ctx *ctx, const b200la_precond *P, SyncFreePlan *plan)
+{
+    constexpr int R = PackRec<T, KP, SGS>::bytes, cap = pack_rows(KP);
+    std::vector<PackTile> tiles;
+    size_t off = 0;
+    int widest = 1;
+    auto add = [&](int r0, int m) {
+        PackTile t{};
+        t.row0 = r0;
+        t.m = m;
+        t.off16 = (unsigned)(off / 16);
+        off += 16 + (size_t)m * R;
+        widest = std::max(widest, m);
+        tiles.push_back(t);
+    };
+    for (int l = 0; l < P->nblocks; ++l)
+        for (int r = P->block_off[l]; r < P->block_off[l + 1]; r += cap) add(r, std::min(cap, P->block_off[l + 1] - r));
+    const int nf = (int)tiles.size();
+    for (int l = P->nblocks - 1; l >= 0; --l)   // rows strictly descending by tile
+        for (int e = P->block_off[l + 1]; e > P->block_off[l]; e -= cap) {
+            const int r = std::max(P->block_off[l], e - cap);
+            add(r, e - r);
+        }
+    if (off / 16 > 0xffffffffull) return cudaSuccess;
+    const int nt = (int)tiles.size(), threads = (widest + 31) / 32 * 32;
+    const int own_off = 16 + threads * R, stage = (own_off + (int)sizeof(T) * threads + 32 + 127) & ~127;
+    const int stages = (int)std::min<size_t>(kPackMaxStages, (kPackSmemCap - pack_head_bytes<T>()) / stage);
+    if (stages < kPackMinStages) return cudaSuccess;
+    cudaError_t e;
+    const size_t tb = sizeof(PackTile) * nt;
+    if ((e = cudaMalloc(&plan->ptiles, tb)) || (e = cudaMemcpy(plan->ptiles, tiles.data(), tb, cudaMemcpyHostToDevice)))
+        return e;
+    pack_far_kernel<<<(nt + 3) / 4, 128, 0, ctx->stream>>>(nt, nf, plan->ptiles, P->L->row, P->L->col, P->U->row,
+                                                           P->U->col, 0, nullptr);
+    if ((e = cudaGetLastError()) ||
+        (e = cudaMemcpyAsync(tiles.data(), plan->ptiles, tb, cudaMemcpyDeviceToHost, ctx->stream)) ||
+        (e = cudaStreamSynchronize(ctx->stream)))
+        return e;
+    long long nfar = 0;
+    for (PackTile &t : tiles) {
+        if (t.nfar > kPackFar || nfar > INT_MAX - 64) return cudaSuccess;
+        t.far0 = (int)nfar;
+        nfar += t.nfar;
+    }
+    if ((e = cudaMemcpy(plan->ptiles, tiles.data(), tb, cudaMemcpyHostToDevice)) ||
+        (e = cudaMalloc(&plan->far, sizeof(int) * std::max<long long>(nfar, 1))) ||
+        (e = cudaMalloc(&plan->pack, std::max<size_t>(off, 16))))
+        return e;
+    pack_far_kernel<<<(nt + 3) / 4, 128, 0, ctx->stream>>>(nt, nf, plan->ptiles, P->L->row, P->L->col, P->U->row,
+                                                           P->U->col, 1, plan->far);
+    pack_tiles_kernel<T, KP, SGS><<<(nt + 3) / 4, 128, 0, ctx->stream>>>(
+        nt, nf, plan->ptiles, P->L->row, P->L->col, (const T *)P->L->val, P->U->row, P->U->col, (const T *)P->U->val,
+        (const T *)P->iDv, (const T *)P->Dv, stages, plan->pack);
+    if ((e = cudaGetLastError()) || (e = cudaStreamSynchronize(ctx->stream))) return e;
+    plan->threads = threads;
+    plan->nf_tiles = nf;
+    plan->nt_tiles = nt;
+    plan->stages = stages;
+    plan->stage_bytes = stage;
+    plan->own_off = own_off;
+    plan->nfar = (int)nfar;
+    plan->kp = KP;
+    return cudaSuccess;
+}
+
+template <typename T, int KP, bool SGS>
+static cudaError_t packed_launch(const SyncFreePlan *plan, const PackedSweepArgs &a, cudaStream_t st)
+{
+    const size_t sm = pack_head_bytes<T>() + (size_t)plan->stages * plan->stage_bytes;
+    level_sweep_packed_kernel<T, KP, SGS><<<1, plan->threads + 32 * (1 + kPackProducers), sm, st>>>(a);
+    return cudaGetLastError();
+}
+
+// f(type, entries, sgs) for the packed kernel instance of P with kp entries per row
+template <class F>
+static cudaError_t packed_dispatch(const b200la_precond *P, int kp, F f)
+{
+    auto by_kp = [&](auto t, auto sgs) {
+        using I4 = std::integral_constant<int, 4>;
+        using I8 = std::integral_constant<int, 8>;
+        using I16 = std::integral_constant<int, 16>;
+        return kp == 4 ? f(t, I4(), sgs) : kp == 8 ? f(t, I8(), sgs) : f(t, I16(), sgs);
+    };
+    auto by_type = [&](auto sgs) { return P->dtype == B200LA_F64 ? by_kp(double(), sgs) : by_kp(float(), sgs); };
+    return P->kind == B200LA_PRECOND_MCSGS ? by_type(std::true_type()) : by_type(std::false_type());
+}
+
 int syncfree_setup(b200la_ctx *ctx, b200la_precond *P)
 {
     const char *env = std::getenv("B200LA_SYNCFREE");
     bool use = P->nblocks > 64;
     if (env) use = std::atoi(env) != 0;
     if (!use) return B200LA_OK;
-    // many small levels: one CTA walks them, with the async-copy look-ahead
-    // when every row of L and U fits kStagedSlots slots (B200LA_SWEEP =
-    // staged / cta / tickets to force a variant)
-    auto maxlen = [](const b200la_csr *M) {
-        int m = 0;
-        for (int i = 0; i < M->n; ++i) m = std::max(m, M->h_row[i + 1] - M->h_row[i]);
-        return m;
-    };
+    // many small levels: one CTA walks them, on the packed stream when the
+    // operator fits it (B200LA_SWEEP = staged / cta / tickets to force a variant)
     const bool few = P->nblocks > 64 && P->n / std::max(P->nblocks, 1) <= 4 * kLevelThreads;
-    int widest = 1;
-    for (int l = 0; l < P->nblocks; ++l) widest = std::max(widest, P->block_off[l + 1] - P->block_off[l]);
-    const int nt = std::min(kLevelThreads, (widest + 31) / 32 * 32);
-    const bool can_stage = P->nblocks <= kStagedMaxLevels && maxlen(P->L) <= kStagedSlots &&
-                           maxlen(P->U) <= kStagedSlots &&
-                           staged_smem<double, kStagedSlots>(P->nblocks, nt) <= kStagedSmemCap;
-    bool cta = few && P->nblocks <= kLevelMaxLevels, staged = few && can_stage;
+    bool cta = few && P->nblocks <= kLevelMaxLevels, staged = few;
     if (const char *sw = std::getenv("B200LA_SWEEP")) {
-        staged = std::strcmp(sw, "staged") == 0 && can_stage;
-        cta = (std::strcmp(sw, "cta") == 0 || std::strcmp(sw, "staged") == 0) && P->nblocks <= kLevelMaxLevels;
+        staged = std::strcmp(sw, "staged") == 0;
+        cta = (std::strcmp(sw, "cta") == 0 || staged) && P->nblocks <= kLevelMaxLevels;
     }
-    if (cta) {
+    if (cta || staged) {
         SyncFreePlan *plan = new SyncFreePlan();
-        plan->nlev = P->nblocks;
-        plan->threads = nt;
-        cudaError_t e;
-        if ((e = cudaMalloc(&plan->lev_off, sizeof(int) * (P->nblocks + 1))) ||
-            (e = cudaMemcpy(plan->lev_off, P->block_off.data(), sizeof(int) * (P->nblocks + 1),
-                            cudaMemcpyHostToDevice))) {
-            if (plan->lev_off) cudaFree(plan->lev_off);
-            delete plan;
+        P->syncfree_plan = plan;
+        cudaError_t e = cudaSuccess;
+        int len = 0;
+        for (const b200la_csr *M : {P->L, P->U})
+            for (int i = 0; i < M->n; ++i) len = std::max(len, M->h_row[i + 1] - M->h_row[i]);
+        if (staged && len <= kPackMaxEntries)
+            e = packed_dispatch(P, len <= 4 ? 4 : len <= 8 ? 8 : 16, [&](auto t, auto kp, auto sgs) {
+                return packed_setup<decltype(t), decltype(kp)::value, decltype(sgs)::value>(ctx, P, plan);
+            });
+        if (e == cudaSuccess && !plan->kp && cta) {
+            plan->nlev = P->nblocks;
+            if (!(e = cudaMalloc(&plan->lev_off, sizeof(int) * (P->nblocks + 1))))
+                e = cudaMemcpy(plan->lev_off, P->block_off.data(), sizeof(int) * (P->nblocks + 1),
+                               cudaMemcpyHostToDevice);
+        }
+        if (e != cudaSuccess) {
+            syncfree_free(P);
             return ctx_fail(ctx, B200LA_ERR_ALLOC, "level sweep setup", e);
         }
-        if (staged) {
-            const size_t es = P->dtype == B200LA_F64 ? 8 : 4, n = (size_t)P->n;
-            for (int m = 0; m < 2 && e == cudaSuccess; ++m) {
-                const b200la_csr *M = m ? P->U : P->L;
-                if ((e = cudaMalloc(&plan->pcol[m], sizeof(int) * kStagedSlots * n)) ||
-                    (e = cudaMalloc(&plan->pval[m], es * kStagedSlots * n)) ||
-                    (e = cudaMalloc(&plan->pcnt[m], sizeof(int) * n)))
-                    break;
-                const int g = std::max(1, std::min((P->n + 255) / 256, 148 * 16));
-                if (P->dtype == B200LA_F64)
-                    pack_rows_kernel<double><<<g, 256, 0, ctx->stream>>>(P->n, kStagedSlots, M->row, M->col,
-                                                                         (const double *)M->val, plan->pcol[m],
-                                                                         (double *)plan->pval[m], plan->pcnt[m]);
-                else
-                    pack_rows_kernel<float><<<g, 256, 0, ctx->stream>>>(P->n, kStagedSlots, M->row, M->col,
-                                                                        (const float *)M->val, plan->pcol[m],
-                                                                        (float *)plan->pval[m], plan->pcnt[m]);
-                e = cudaGetLastError();
-            }
-            if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-            if (e != cudaSuccess) {
-                P->syncfree_plan = plan;
-                syncfree_free(P);
-                return ctx_fail(ctx, B200LA_ERR_ALLOC, "staged level sweep setup", e);
-            }
-            plan->staged = 1;
+        if (plan->kp || plan->lev_off) {
+            P->use_syncfree = 1;
+            return B200LA_OK;
         }
-        P->syncfree_plan = plan;
-        P->use_syncfree = 1;
-        return B200LA_OK;
+        syncfree_free(P);
     }
     const int lgL = lanes_for(P->L), lgU = lanes_for(P->U);
     // chunks of at most 32 >> lg rows, never crossing a block (level) boundary
@@ -611,11 +890,9 @@ void syncfree_free(b200la_precond *P)
     if (plan->fwd) cudaFree(plan->fwd);
     if (plan->bwd) cudaFree(plan->bwd);
     if (plan->lev_off) cudaFree(plan->lev_off);
-    for (int m = 0; m < 2; ++m) {
-        if (plan->pcol[m]) cudaFree(plan->pcol[m]);
-        if (plan->pval[m]) cudaFree(plan->pval[m]);
-        if (plan->pcnt[m]) cudaFree(plan->pcnt[m]);
-    }
+    if (plan->ptiles) cudaFree(plan->ptiles);
+    if (plan->far) cudaFree(plan->far);
+    if (plan->pack) cudaFree(plan->pack);
     delete plan;
     P->syncfree_plan = nullptr;
 }
@@ -623,33 +900,27 @@ void syncfree_free(b200la_precond *P)
 int syncfree_apply(b200la_ctx *ctx, const b200la_precond *P, const void *r, void *z, const int *gate)
 {
     const SyncFreePlan *plan = static_cast<const SyncFreePlan *>(P->syncfree_plan);
-    if (plan->staged) {
-        LevelStagedArgs a;
-        a.off = plan->lev_off;
-        a.nlev = plan->nlev;
+    if (plan->kp) {
+        PackedSweepArgs a;
+        a.tiles = plan->ptiles;
+        a.pack = plan->pack;
+        a.far = plan->far;
+        a.nfar = plan->nfar;
+        a.nf = plan->nf_tiles;
+        a.nt = plan->nt_tiles;
         a.n = P->n;
+        a.stages = plan->stages;
+        a.stage_bytes = plan->stage_bytes;
+        a.own_off = plan->own_off;
         a.r = r;
         a.z = z;
-        a.d1 = P->iDv;
-        a.d2 = P->Dv;
-        a.sgs = P->kind == B200LA_PRECOND_MCSGS;
         a.gate = gate;
-        for (int dir = 0; dir < 2; ++dir) {
-            a.pcol = plan->pcol[dir];
-            a.pval = plan->pval[dir];
-            a.pcnt = plan->pcnt[dir];
-            a.backward = dir;
-            const int nt = plan->threads;
-            if (P->dtype == B200LA_F64)
-                level_sweep_staged_kernel<double, kStagedSlots>
-                    <<<1, nt, staged_smem<double, kStagedSlots>(plan->nlev, nt), ctx->stream>>>(a);
-            else
-                level_sweep_staged_kernel<float, kStagedSlots>
-                    <<<1, nt, staged_smem<float, kStagedSlots>(plan->nlev, nt), ctx->stream>>>(a);
-            cudaError_t e = cudaGetLastError();
-            if (e != cudaSuccess) return ctx_fail(ctx, B200LA_ERR_CUDA, "staged level sweep", e);
-            ctx->launches += 1;
-        }
+        a.err = ctx->dev_err;
+        const cudaError_t e = packed_dispatch(P, plan->kp, [&](auto t, auto kp, auto sgs) {
+            return packed_launch<decltype(t), decltype(kp)::value, decltype(sgs)::value>(plan, a, ctx->stream);
+        });
+        if (e != cudaSuccess) return ctx_fail(ctx, B200LA_ERR_CUDA, "packed level sweep", e);
+        ctx->launches += 1;
         return B200LA_OK;
     }
     if (plan->lev_off) {

@@ -378,6 +378,44 @@ def test_captured_graphs_follow_new_objects(pf, b200):
             ref = sl.spsolve(sp.csc_matrix(sp.csr_matrix((val * scale, col, row), shape=(n, n))), bh)
             assert np.linalg.norm(x.numpy() - ref) <= 1e-8 * np.linalg.norm(ref)
         del P, A, gm, cg
+@pytest.mark.parametrize("dim,N,p,dtype", [(2, 2, 0, 0), (2, 33, 0, 0), (2, 33, 0, 1), (2, 40, 1, 0), (2, 40, 1, 1),
+                                           (3, 7, 0, 0), (2, 70, 2, 0), (2, 1100, 0, 0)])
+def test_level_sweep_packed_edges(pf, b200, dim, N, p, dtype, monkeypatch):
+    """The packed level sweep against substitution with the host's factors
+    (couplings inside a level dropped, as the block preconditioner does):
+    levels of one row, ragged levels, more than one tile per level (N = 1100),
+    4 / 8 / 16 entries per row, vectors that start and end inside a 16-byte
+    unit.  Bars: FP64 1e-12 of the largest entry (the applies'
+    bar), FP32 2e-5 (about 300 roundings of 6e-8)."""
+    import scipy.sparse as sp
+    import scipy.sparse.linalg as sl
+    torch = pytest.importorskip("torch")
+    row, col, val = b200.q1_assemble(dim, N, 1, None, 1e-2, (1.0, 0.5, 0.25))
+    n = len(row) - 1
+    fr, fc, fv = (row, col, b200.ilu0(row, col, val)) if p == 0 else b200.ilup(row, col, val, p)
+    F = sp.csr_matrix((fv, fc, fr), shape=(n, n))
+    r = np.random.default_rng(N).uniform(-1, 1, n)
+    monkeypatch.setenv("B200LA_SYNCFREE", "1")
+    monkeypatch.setenv("B200LA_SWEEP", "staged")
+    P = b200.Preconditioner.ILU0(pf, row, col, val, b200.PRECOND_ILU0_LS, dtype) if p == 0 else \
+        b200.Preconditioner.ILUp(pf, row, col, val, p, mode=b200.PRECOND_ILU0_LS, dtype=dtype)
+    F = F[P.perm][:, P.perm].tocoo()
+    level = np.repeat(np.arange(P.nblocks), P.block_sizes)
+    keep = (level[F.row] != level[F.col]) | (F.row == F.col)
+    F = sp.csr_matrix((F.data[keep], (F.row[keep], F.col[keep])), shape=(n, n))
+    rp, tol = r[P.perm], 2e-5 if dtype else 1e-12
+    L = sp.tril(F, -1, format="csr") + sp.identity(n, format="csr")
+    ref = sl.spsolve_triangular(sp.triu(F, 0, format="csr"), sl.spsolve_triangular(L, rp, lower=True), lower=False)
+    td = torch.float32 if dtype else torch.float64
+    for shift in (0, 1):
+        with pf.on_stream():
+            buf = torch.full((2, n + 8), 7.0, dtype=td, device="cuda")
+            buf[0, shift:shift + n] = torch.from_numpy(rp).to(buf)
+        vr, vz = (b200.lVector(pf, buf[k, shift:shift + n]) for k in (0, 1))
+        P.ApplyPreconditioner(vr, vz)
+        assert np.max(np.abs(vz.numpy() - ref)) <= tol * np.max(np.abs(ref))
+        edges = torch.cat([buf[:, :shift], buf[:, shift + n:]], 1)
+        assert bool((edges == 7.0).all())
 
 
 @pytest.mark.parametrize("precond", ["none", "jacobi", "mcsgs"])
