@@ -45,6 +45,7 @@ struct b200la_ctx {
     double *partials = nullptr;     // grid-reduction partials [8][kMaxGrid]
     unsigned *ticket = nullptr;     // last-CTA tickets
     int *dev_err = nullptr;         // device error flag (bounded waits)
+    unsigned char *gather = nullptr;   // words of the cooperative kernels' grid sums (grid_gather.cuh)
     b200::DevState *st = nullptr;   // device solver state
     b200::DevState *st_host = nullptr;   // pinned mirror
     double *dscal = nullptr;        // device scalars (256)

@@ -6,6 +6,7 @@
 // kernels.cu / sweeps.cu; there is no host fallback.
 #include "b200la.h"
 #include "b200la_internal.h"
+#include "grid_gather.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -187,6 +188,7 @@ extern "C" int b200la_create(int device, b200la_ctx **out)
     if ((e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking)) ||
         (e = cudaMalloc(&ctx->partials, sizeof(double) * 8 * kMaxGrid)) ||
         (e = cudaMalloc(&ctx->ticket, sizeof(unsigned) * kTicketWords)) || (e = cudaMalloc(&ctx->dev_err, sizeof(int))) ||
+        (e = cudaMalloc(&ctx->gather, kGatherBytes)) || (e = cudaMemset(ctx->gather, 0, kGatherBytes)) ||
         (e = cudaMalloc(&ctx->st, sizeof(DevState))) || (e = cudaMalloc(&ctx->dscal, sizeof(double) * 256)) ||
         (e = cudaMallocHost(&ctx->st_host, sizeof(DevState))) ||
         (e = cudaMallocHost(&ctx->hscal, sizeof(double) * 256)) || (e = cudaEventCreate(&ctx->ev0)) ||
@@ -212,6 +214,7 @@ extern "C" int b200la_destroy(b200la_ctx *ctx)
     if (ctx->partials) cudaFree(ctx->partials);
     if (ctx->ticket) cudaFree(ctx->ticket);
     if (ctx->dev_err) cudaFree(ctx->dev_err);
+    if (ctx->gather) cudaFree(ctx->gather);
     if (ctx->st) cudaFree(ctx->st);
     if (ctx->dscal) cudaFree(ctx->dscal);
     if (ctx->st_host) cudaFreeHost(ctx->st_host);

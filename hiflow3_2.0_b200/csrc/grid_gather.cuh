@@ -51,7 +51,7 @@ template <int THREADS>
 struct GridGather {
     static_assert(THREADS >= kGatherMaxCtas, "one thread per CTA's word");
     struct Shared {
-        double part[kGatherMaxQ][THREADS / 32], total[kGatherMaxQ];
+        double part[kGatherMaxQ][THREADS / 32], tot[kGatherMaxQ][kGatherMaxCtas / 32];
         int fail;
     };
     unsigned char *words;
@@ -115,19 +115,18 @@ struct GridGather {
                 }
             }
         }
-        // the partials of part[] were consumed before the words were published
         if (warp * 32 < ctas) {
 #pragma unroll
             for (int q = 0; q < NQ; ++q) {
                 const double w = warp_sum(v[q]);
-                if (lane == 0) sh.total_part(q, warp) = w;
+                if (lane == 0) sh.tot[q][warp] = w;
             }
         }
         __syncthreads();
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {
             double s = 0.0;
-            for (int w = 0; w * 32 < ctas; ++w) s += sh.total_part(q, w);
+            for (int w = 0; w * 32 < ctas; ++w) s += sh.tot[q][w];
             out[q] = s;
         }
     }

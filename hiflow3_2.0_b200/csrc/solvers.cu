@@ -11,12 +11,14 @@
 // exactly those of IterateControl::Check (src/common/iterate_control.cc:84-110).
 #include "b200la.h"
 #include "b200la_internal.h"
+#include "grid_gather.cuh"
 
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 using namespace b200;
@@ -611,6 +613,184 @@ __global__ void gmres_givens_kernel(int j, int m, GmresDev d, DevState *st)
     if (s != kIterate) *d.jend = j;
 }
 
+// Modified Gram-Schmidt of one Arnoldi step (gmres.cc:373-402) in one launch:
+// w stays in registers (EV 16-byte vectors per thread), every product sums over
+// the grid by a gather (grid_gather.cuh), v_{i+1} is loaded while the sum of
+// v_i travels, the norm, V_{j+1} = w / ||w||, the Givens rotations (on CTA 0,
+// while it waits) and the check follow in the same launch.
+//   Bound by the j + 2 grid sums: the basis lies in L2 at these sizes.  A dot
+// and an axpy launch per basis vector took 8.5 us at 2-D 512^2 (2.1 MB per
+// vector).  GMRES(30) + ILU(0) 512^2 to 1e-10: 170 -> 145 ms; mixed 300^2: 25.8
+// -> 20.9 ms; ILU(1) 200^2: 9.8 -> 8.3 ms.  The launches stay for vectors that
+// do not fit the registers of one CTA per SM (1.2 million doubles), where their
+// bytes outweigh the launches.
+constexpr int kOrthThreads = 512;
+
+template <typename T, int EV>
+__global__ void __launch_bounds__(kOrthThreads) gmres_orth_kernel(int n, int j, int m, const T *__restrict__ w,
+                                                                  T *__restrict__ V, size_t ld, GmresDev d,
+                                                                  DevState *st, unsigned char *gmem, int *err)
+{
+    if (gate_closed(&st->status)) return;
+    using V4 = std::conditional_t<sizeof(T) == 8, double2, float4>;
+    constexpr int W = 16 / (int)sizeof(T);
+    __shared__ typename GridGather<kOrthThreads>::Shared sh;
+    GridGather<kOrthThreads> gg(gmem, sh, err);
+    const int stride = gridDim.x * kOrthThreads, first = blockIdx.x * kOrthThreads + threadIdx.x;
+    const bool scribe = blockIdx.x == 0 && threadIdx.x == 0;
+    double *Hj = d.H + (size_t)j * (m + 1);
+    struct Vec {
+        T e[W];
+    };
+    // vector iv of a basis vector, entries past n as zero (the vectors are padded to 256 bytes)
+    auto load = [&](const T *p, Vec (&q)[EV]) {
+#pragma unroll
+        for (int u = 0; u < EV; ++u) {
+            const int iv = first + u * stride;
+            V4 t = {};
+            if ((long long)iv * W < n) t = *reinterpret_cast<const V4 *>(p + (size_t)iv * W);
+            q[u].e[0] = t.x;
+            q[u].e[1] = t.y;
+            if constexpr (W == 4) {
+                q[u].e[2] = t.z;
+                q[u].e[3] = t.w;
+            }
+#pragma unroll
+            for (int k = 1; k < W; ++k)
+                if ((long long)iv * W + k >= n) q[u].e[k] = T(0);
+        }
+    };
+    auto dot = [&](const Vec (&a)[EV], const Vec (&b)[EV]) {
+        double s = 0.0;
+#pragma unroll
+        for (int u = 0; u < EV; ++u) {
+            T t = T(0);
+#pragma unroll
+            for (int k = 0; k < W; ++k) t += a[u].e[k] * b[u].e[k];
+            s += (double)t;
+        }
+        return s;
+    };
+    Vec x[EV], v[EV], vn[EV] = {};
+    load(w, x);
+    load(V, v);
+    // rotation k of the column (gmres.h:77-97), once H(j, k) and H(j, k + 1) are known
+    double hk = 0.0;   // scribe: H(j, k) after the rotations before k
+    auto rotate = [&](int k, double next) {
+        const double t = d.cs[k] * hk + d.sn[k] * next;
+        const double r = -d.sn[k] * hk + d.cs[k] * next;
+        Hj[k] = t;
+        hk = r;
+    };
+    double hlast = 0.0;   // H(j, i - 1), not yet rotated
+    for (int i = 0; i <= j; ++i) {
+        const double part[1] = {dot(x, v)};
+        gg.template publish<1, false>(part);
+        if (i < j) load(V + (size_t)(i + 1) * ld, vn);
+        if (scribe) {
+            if (i == 1) hk = hlast;
+            if (i > 1) rotate(i - 2, hlast);
+        }
+        double h[1];
+        gg.template total<1, false>(h);
+        const T c = (T)(-1.0 * h[0]);
+#pragma unroll
+        for (int u = 0; u < EV; ++u) {
+#pragma unroll
+            for (int k = 0; k < W; ++k) {
+                x[u].e[k] += c * v[u].e[k];
+                v[u].e[k] = vn[u].e[k];
+            }
+        }
+        hlast = h[0];
+    }
+    const double part[1] = {dot(x, x)};
+    gg.template publish<1, false>(part);
+    if (scribe) {
+        if (j == 0) hk = hlast;
+        else rotate(j - 1, hlast);
+    }
+    double nn[1];
+    gg.template total<1, false>(nn);
+    const double norm = sqrt(nn[0]);
+    gg.close();
+    // V_{j+1} = w / H(j, j+1)
+    const T c = (T)(1.0 / norm);
+    T *out = V + (size_t)(j + 1) * ld;
+#pragma unroll
+    for (int u = 0; u < EV; ++u) {
+        const int iv = first + u * stride;
+        if ((long long)iv * W + W <= n) {
+            V4 t;
+            t.x = c * x[u].e[0];
+            t.y = c * x[u].e[1];
+            if constexpr (W == 4) {
+                t.z = c * x[u].e[2];
+                t.w = c * x[u].e[3];
+            }
+            *reinterpret_cast<V4 *>(out + (size_t)iv * W) = t;
+        } else {
+#pragma unroll
+            for (int k = 0; k < W; ++k)
+                if ((long long)iv * W + k < n) out[(size_t)iv * W + k] = c * x[u].e[k];
+        }
+    }
+    if (!scribe) return;
+    // the new rotation (gmres.cc:380-402)
+    const double beta = sqrt(hk * hk + norm * norm);
+    const double cs = hk / beta, sn = norm / beta;
+    d.cs[j] = cs;
+    d.sn[j] = sn;
+    Hj[j] = cs * hk + sn * norm;
+    Hj[j + 1] = -sn * hk + cs * norm;
+    const double gj = d.g[j], gn = d.g[j + 1];
+    d.g[j + 1] = -sn * gj + cs * gn;
+    d.g[j] = cs * gj + sn * gn;
+    const double res = fabs(d.g[j + 1]);
+    const int it = st->iter + 1;
+    st->iter = it;
+    st->res = res;
+    const int s = check_dev(st, it, res);
+    st->status = s;
+    if (s != kIterate) *d.jend = j;
+}
+
+// CTAs of the one-launch orthogonalisation for vectors of n entries, and the
+// 16-byte vectors per thread; 0: they do not fit.
+static int orth_grid(int n, size_t es, int num_sms, int *ev)
+{
+    const long long nv = ((long long)n * (long long)es + 15) / 16;
+    const int cap = std::min(num_sms, kGatherMaxCtas);
+    for (int e = 1; e <= 8; e *= 2)
+        if (nv <= (long long)cap * kOrthThreads * e) {
+            *ev = e;
+            return (int)std::max(1LL, (nv + (long long)kOrthThreads * e - 1) / ((long long)kOrthThreads * e));
+        }
+    return 0;
+}
+
+template <typename T>
+static cudaError_t launch_gmres_orth(int grid, int ev, int n, int j, int m, const void *w, void *V, size_t ld, GmresDev d,
+                                     DevState *st, unsigned char *gmem, int *err, cudaStream_t stream)
+{
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = kOrthThreads;
+    cfg.stream = stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    auto go = [&](auto kern) { return cudaLaunchKernelEx(&cfg, kern, n, j, m, (const T *)w, (T *)V, ld, d, st, gmem, err); };
+    switch (ev) {
+    case 1: return go(gmres_orth_kernel<T, 1>);
+    case 2: return go(gmres_orth_kernel<T, 2>);
+    case 4: return go(gmres_orth_kernel<T, 4>);
+    default: return go(gmres_orth_kernel<T, 8>);
+    }
+}
+
 // Back substitution of UpdateSolution (gmres.cc:487-504) into y[0..k].
 __global__ void gmres_backsub_kernel(int k, int m, GmresDev d)
 {
@@ -680,6 +860,8 @@ extern "C" int b200la_gmres(b200la_ctx *ctx, const b200la_csr *A, const b200la_p
     const Scratch sc = ctx_scratch(ctx);
     const long long l0 = ctx->launches;
     const size_t ld_el = ldv / es;
+    int ev = 0;
+    const int orth = orth_grid(n, es, ctx->num_sms, &ev);
 
     DevState *hs = ctx->st_host;
     state_init(*hs, ctl, nullptr, 0);
@@ -720,6 +902,14 @@ extern "C" int b200la_gmres(b200la_ctx *ctx, const b200la_csr *A, const b200la_p
                 o.gate = gate;
                 int r2 = spmv_run(ctx, A, A->all, o);
                 if (r2) return r2;
+                if (orth) {
+                    SK(dt == B200LA_F64 ? launch_gmres_orth<double>(orth, ev, n, j, mb, w, V(0), ld_el, d, ctx->st,
+                                                                    ctx->gather, ctx->dev_err, ctx->stream)
+                                        : launch_gmres_orth<float>(orth, ev, n, j, mb, w, V(0), ld_el, d, ctx->st,
+                                                                   ctx->gather, ctx->dev_err, ctx->stream));
+                    ctx->launches += 1;
+                    continue;
+                }
                 // modified Gram-Schmidt (gmres.cc:373-377)
                 for (int i = 0; i <= j; ++i) {
                     SK(launch_dot_to(sc, dt, n, w, V(i), d.H + (size_t)j * (mb + 1) + i, gate, ctx->stream));

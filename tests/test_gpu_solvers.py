@@ -340,6 +340,60 @@ def test_ilu0_level_sweep_beyond_ring(pf, b200, dim, N, kind, monkeypatch):
 
 
 
+@pytest.mark.parametrize("n,dtype", [(1, 0), (2, 0), (511, 0), (1025, 1), (4097, 0), (151553, 0), (151553, 1),
+                                     (303107, 0), (606211, 1), (640000, 0)])
+def test_gmres_one_launch_orthogonalisation(pf, b200, n, dtype):
+    """GMRES(5) on a tridiagonal operator at sizes around the vectors a thread
+    holds (one to eight 16-byte ones, the last ragged, one CTA to all): the
+    same steps and the iterate of a host GMRES(5), within 1e-10 (FP64: ~20
+    steps of roundings of 1e-16 amplified by the residual's fall of 1e3) or
+    1e-4 (FP32) of the largest entry."""
+    rng = np.random.default_rng(n)
+    m = min(5, n)
+    i = np.arange(n)
+    lo, up = -rng.uniform(0.2, 0.6, n), -rng.uniform(0.2, 0.6, n)
+    c = np.stack([i - 1, i, i + 1], 1)
+    v = np.stack([lo, np.full(n, 2.0), up], 1)
+    keep = (c >= 0) & (c < n)
+    row = np.concatenate([[0], np.cumsum(keep.sum(1))]).astype(np.int32)
+    A = b200.CSR_lMatrix.from_csr(pf, row, c[keep].astype(np.int32), v[keep], dtype=dtype)
+    bh = rng.uniform(-1, 1, n)
+
+    def mult(x):
+        y = 2.0 * x
+        y[1:] += lo[1:] * x[:-1]
+        y[:-1] += up[:-1] * x[1:]
+        return y
+
+    x, steps = np.zeros(n), 0
+    for _ in range(2):
+        r = bh - mult(x)
+        beta = np.linalg.norm(r)
+        V, H = [r / beta], np.zeros((m + 1, m))
+        for j in range(m):
+            w = mult(V[j])
+            for k in range(j + 1):
+                H[k, j] = w @ V[k]
+                w = w - H[k, j] * V[k]
+            H[j + 1, j] = np.linalg.norm(w)
+            if H[j + 1, j] < 1e-14:
+                break
+            V.append(w / H[j + 1, j])
+        k = j + 1
+        y = np.linalg.lstsq(H[:k + 1, :k], np.eye(k + 1)[0] * beta, rcond=None)[0]
+        x = x + np.stack(V[:k], 1) @ y
+        steps += k
+        if n <= 5:
+            break
+    gm = b200.GMRES(pf, m)
+    gm.SetupOperator(A)
+    gm.InitControl(steps, 0.0, 1e-14 if n > 5 else 1e-9, 1e6)
+    xv = pf.vector(n, dtype)
+    gm.Solve(pf.vector(bh, dtype), xv)
+    assert gm.iter() <= steps
+    assert np.max(np.abs(xv.numpy() - x)) <= (1e-4 if dtype else 1e-10) * np.max(np.abs(x))
+
+
 def test_captured_graphs_follow_new_objects(pf, b200):
     """A solve after its operator and preconditioner were freed and others made
     (whose handles may get the freed addresses again) runs on the new ones: the
