@@ -18,6 +18,7 @@ struct NvtxScope {
     NvtxScope &operator=(const NvtxScope &) = delete;
 };
 
+#include "b200la.h"
 #include "common.cuh"
 #include "host_setup.h"
 #include "kernels.cuh"
@@ -46,6 +47,7 @@ struct b200la_ctx {
     unsigned *ticket = nullptr;     // last-CTA tickets
     int *dev_err = nullptr;         // device error flag (bounded waits)
     unsigned char *gather = nullptr;   // words of the cooperative kernels' grid sums (grid_gather.cuh)
+    void *rows = nullptr;           // row words of the one-launch CG (made at its first solve)
     b200::DevState *st = nullptr;   // device solver state
     b200::DevState *st_host = nullptr;   // pinned mirror
     double *dscal = nullptr;        // device scalars (256)
@@ -145,6 +147,10 @@ int syncfree_apply(b200la_ctx *ctx, const b200la_precond *P, const void *r, void
 void syncfree_free(b200la_precond *P);
 // solvers.cu
 void graph_cache_clear(b200la_ctx *ctx);
+// cg_fused.cu
+int cg_fused_rows(const b200la_ctx *ctx, const b200la_csr *A);
+cudaError_t cg_fused_run(b200la_ctx *ctx, const b200la_csr *A, const void *invd, const void *b, void *x,
+                         const b200la_control *ctl, double *hist, int hist_len, int rows);
 // lattice.cu
 namespace lattice {
 bool grid(int n, const int *row, const int *col, int *mx, int *my, int *mz);

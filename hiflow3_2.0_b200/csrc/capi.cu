@@ -215,6 +215,7 @@ extern "C" int b200la_destroy(b200la_ctx *ctx)
     if (ctx->ticket) cudaFree(ctx->ticket);
     if (ctx->dev_err) cudaFree(ctx->dev_err);
     if (ctx->gather) cudaFree(ctx->gather);
+    if (ctx->rows) cudaFree(ctx->rows);
     if (ctx->st) cudaFree(ctx->st);
     if (ctx->dscal) cudaFree(ctx->dscal);
     if (ctx->st_host) cudaFreeHost(ctx->st_host);

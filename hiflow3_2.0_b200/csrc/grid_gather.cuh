@@ -1,18 +1,20 @@
 // grid_gather.cuh -- sums over the whole grid inside one cooperative launch.
 //
 // A solver step whose vectors fit the chip spends its time on launches and
-// reduction tails, not on bytes.  Here every CTA publishes its partial sum and
-// the epoch of the sum as one 16-byte word, and every CTA polls the words of
-// all CTAs until they carry that epoch: one L2 write and one L2 read stand
-// between a partial and its total (about 1 us over 148 CTAs), where a ticket
-// barrier takes an atomic, a flag and the read of the partials behind it, and
-// a kernel boundary several microseconds.  All CTAs add the partials in the
-// same order, so they hold the same bits and take the same decisions.
+// reduction tails, not on bytes.  Here every CTA writes its partial sum and the
+// epoch of the sum as one 16-byte word, and every CTA polls the words of all
+// CTAs until they carry that epoch: one trip through L2 stands between a partial
+// and its total, no atomic and no fence, where a kernel boundary costs several
+// microseconds.  All CTAs add the partials in the same order, so they hold the
+// same bits and take the same decisions.  A word has a line of its own: words
+// that share a line, copies of the words, a mailbox per reader, and a CTA that
+// collects and hands out the total (two trips) were all slower (per iteration of
+// a CG with two sums, 130 CTAs: 7.0 us against 10.2, 7.9, 7.5 and 8.6).
 //
 // Epochs rise through the life of the context.  Words are double-buffered by
-// the epoch's parity: a CTA publishes epoch k + 2 only after every CTA has
-// published k + 1, which each does after it has read k.  Polls are bounded;
-// after one has run out (reported in the error flag) nothing waits any more.
+// the epoch's parity: a CTA writes epoch k + 2 only after it has seen k + 1 of
+// every CTA, which each writes after it has read k.  Polls are bounded; after
+// one has run out (reported in the error flag) nothing waits any more.
 #pragma once
 
 #include "common.cuh"
@@ -22,26 +24,18 @@ namespace b200 {
 constexpr int kGatherMaxQ = 2;         // quantities per sum
 constexpr int kGatherMaxCtas = 160;    // CTAs of a gathering grid
 constexpr long long kGatherSpin = 1LL << 22;
-constexpr size_t kGatherBytes = 16 + 16 * (size_t)2 * kGatherMaxQ * kGatherMaxCtas;
+constexpr size_t kGatherBytes = 128 * (1 + (size_t)2 * kGatherMaxCtas);   // the last epoch, the words of two epochs
 
-__device__ __forceinline__ void st_word(void *p, double v, unsigned long long e, bool release)
+__device__ __forceinline__ void st_word(void *p, double v, unsigned long long e)
 {
-    if (release)
-        asm volatile("{\n\t.reg .b128 w;\n\tmov.b128 w, {%1, %2};\n\tst.release.gpu.global.b128 [%0], w;\n\t}" ::"l"(p),
-                     "l"(__double_as_longlong(v)), "l"(e) : "memory");
-    else
-        asm volatile("{\n\t.reg .b128 w;\n\tmov.b128 w, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], w;\n\t}" ::"l"(p),
-                     "l"(__double_as_longlong(v)), "l"(e) : "memory");
+    asm volatile("{\n\t.reg .b128 w;\n\tmov.b128 w, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], w;\n\t}" ::"l"(p),
+                 "l"(__double_as_longlong(v)), "l"(e) : "memory");
 }
-__device__ __forceinline__ void ld_word(const void *p, double &v, unsigned long long &e, bool acquire)
+__device__ __forceinline__ void ld_word(const void *p, double &v, unsigned long long &e)
 {
     long long x;
-    if (acquire)
-        asm volatile("{\n\t.reg .b128 w;\n\tld.acquire.gpu.global.b128 w, [%2];\n\tmov.b128 {%0, %1}, w;\n\t}"
-                     : "=l"(x), "=l"(e) : "l"(p) : "memory");
-    else
-        asm volatile("{\n\t.reg .b128 w;\n\tld.relaxed.gpu.global.b128 w, [%2];\n\tmov.b128 {%0, %1}, w;\n\t}"
-                     : "=l"(x), "=l"(e) : "l"(p) : "memory");
+    asm volatile("{\n\t.reg .b128 w;\n\tld.relaxed.gpu.global.b128 w, [%2];\n\tmov.b128 {%0, %1}, w;\n\t}"
+                 : "=l"(x), "=l"(e) : "l"(p) : "memory");
     v = __longlong_as_double(x);
 }
 
@@ -60,7 +54,7 @@ struct GridGather {
     int *err;
 
     // `mem`: kGatherBytes of the context (the last epoch used, then the words)
-    __device__ GridGather(unsigned char *mem, Shared &s, int *e) : words(mem + 16), sh(s), err(e)
+    __device__ GridGather(unsigned char *mem, Shared &s, int *e) : words(mem + 128), sh(s), err(e)
     {
         epoch = __ldcg(reinterpret_cast<const unsigned long long *>(mem));
         if (threadIdx.x == 0) sh.fail = 0;
@@ -69,10 +63,11 @@ struct GridGather {
     // after the last sum, by CTA 0: the next kernel goes on from there
     __device__ void close()
     {
-        if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned long long *>(words - 16) = epoch;
+        if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned long long *>(words - 128) = epoch;
     }
-    // Publish this CTA's sums of v (ORDERED: with everything its threads wrote before).
-    template <int NQ, bool ORDERED>
+    // Publish this CTA's sums of v.  (Nothing else is ordered by it: data that
+    // CTAs exchange carry epochs themselves, as a fence costs about 1 us.)
+    template <int NQ>
     __device__ void publish(const double (&v)[NQ])
     {
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -87,38 +82,19 @@ struct GridGather {
 #pragma unroll
             for (int q = 0; q < NQ; ++q) {
                 const double s = warp_sum(lane < THREADS / 32 ? sh.part[q][lane] : 0.0);
-                if (lane == q) st_word(word(q, blockIdx.x), s, epoch, ORDERED);
+                if (lane == q) st_word(word(blockIdx.x, q), s, epoch);
             }
         }
     }
-    // Totals of the sums published last, in every thread (ORDERED: what the
-    // CTAs wrote before publishing may be read).
-    template <int NQ, bool ORDERED>
+    // Totals of the sums published last, in every thread.
+    template <int NQ>
     __device__ void total(double (&out)[NQ])
     {
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ctas = gridDim.x;
-        double v[NQ];
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) v[q] = 0.0;
-        if ((int)threadIdx.x < ctas) {
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) {
-                unsigned long long e;
-                volatile int *fail = &sh.fail;
-                ld_word(word(q, threadIdx.x), v[q], e, ORDERED);
-                for (long long i = 0; e != epoch && !*fail; ++i) {
-                    if (i > kGatherSpin) {
-                        *fail = 1;
-                        atomicExch(err, kDevWaitTimeout);
-                    }
-                    ld_word(word(q, threadIdx.x), v[q], e, ORDERED);
-                }
-            }
-        }
         if (warp * 32 < ctas) {
 #pragma unroll
             for (int q = 0; q < NQ; ++q) {
-                const double w = warp_sum(v[q]);
+                const double w = warp_sum((int)threadIdx.x < ctas ? poll(word(threadIdx.x, q)) : 0.0);
                 if (lane == 0) sh.tot[q][warp] = w;
             }
         }
@@ -130,11 +106,30 @@ struct GridGather {
             out[q] = s;
         }
     }
+    // after an unsuccessful poll number i: true when to give up
+    __device__ bool stop(long long i)
+    {
+        volatile int *fail = &sh.fail;
+        if (*fail) return true;
+        if (i > kGatherSpin) {
+            *fail = 1;
+            atomicExch(err, kDevWaitTimeout);
+        }
+        return false;
+    }
 
 private:
-    __device__ void *word(int q, int cta)
+    __device__ double poll(const void *p)
     {
-        return words + 16 * (((epoch & 1) * kGatherMaxQ + q) * kGatherMaxCtas + cta);
+        double v;
+        unsigned long long e;
+        ld_word(p, v, e);
+        for (long long i = 0; e != epoch && !stop(i); ++i) ld_word(p, v, e);
+        return v;
+    }
+    __device__ void *word(int cta, int q)
+    {
+        return words + 128 * ((int)(epoch & 1) * kGatherMaxCtas + cta) + 16 * q;
     }
 };
 

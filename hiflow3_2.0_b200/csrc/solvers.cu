@@ -178,6 +178,27 @@ static int cg_core(b200la_ctx *ctx, const b200la_csr *A, const b200la_precond *P
     const Scratch sc = ctx_scratch(ctx);
     const long long l0 = ctx->launches;
 
+    if (const int rows = pc < 2 ? cg_fused_rows(ctx, A) : 0) {
+        DevState *fs = ctx->st_host;
+        if (time_it) SK(cudaEventRecord(ctx->ev0, ctx->stream));
+        SK(cg_fused_run(ctx, A, invd, b, x, ctl, hist_dev, hist_len, rows));
+        if (time_it) SK(cudaEventRecord(ctx->ev1, ctx->stream));
+        SK(cudaStreamSynchronize(ctx->stream));
+        float ms = 0.f;
+        if (time_it) SK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
+        if (fs->pad0 != 0.0)
+            if (const int rc = ctx_check_device_error(ctx)) return rc;
+        if (res) {
+            res->iters = fs->iter;
+            res->status = fs->status;
+            res->res0 = fs->res0;
+            res->res = fs->res;
+            res->outer = 0;
+            res->launches = (int)(ctx->launches - l0);
+            res->solve_ms = ms;
+        }
+        return B200LA_OK;
+    }
     DevState *hs = ctx->st_host;
     state_init(*hs, ctl, hist_dev, hist_len);
     SK(cudaMemcpyAsync(ctx->st, hs, sizeof(DevState), cudaMemcpyHostToDevice, ctx->stream));
@@ -685,14 +706,14 @@ __global__ void __launch_bounds__(kOrthThreads) gmres_orth_kernel(int n, int j, 
     double hlast = 0.0;   // H(j, i - 1), not yet rotated
     for (int i = 0; i <= j; ++i) {
         const double part[1] = {dot(x, v)};
-        gg.template publish<1, false>(part);
+        gg.template publish<1>(part);
         if (i < j) load(V + (size_t)(i + 1) * ld, vn);
         if (scribe) {
             if (i == 1) hk = hlast;
             if (i > 1) rotate(i - 2, hlast);
         }
         double h[1];
-        gg.template total<1, false>(h);
+        gg.template total<1>(h);
         const T c = (T)(-1.0 * h[0]);
 #pragma unroll
         for (int u = 0; u < EV; ++u) {
@@ -705,13 +726,13 @@ __global__ void __launch_bounds__(kOrthThreads) gmres_orth_kernel(int n, int j, 
         hlast = h[0];
     }
     const double part[1] = {dot(x, x)};
-    gg.template publish<1, false>(part);
+    gg.template publish<1>(part);
     if (scribe) {
         if (j == 0) hk = hlast;
         else rotate(j - 1, hlast);
     }
     double nn[1];
-    gg.template total<1, false>(nn);
+    gg.template total<1>(nn);
     const double norm = sqrt(nn[0]);
     gg.close();
     // V_{j+1} = w / H(j, j+1)

@@ -394,6 +394,82 @@ def test_gmres_one_launch_orthogonalisation(pf, b200, n, dtype):
     assert np.max(np.abs(xv.numpy() - x)) <= (1e-4 if dtype else 1e-10) * np.max(np.abs(x))
 
 
+@pytest.mark.parametrize("dim,N,half", [(2, 1, 1), (2, 2, 1), (2, 21, 1), (2, 21, 0), (2, 274, 1), (2, 275, 0), (2, 275, 1),
+                                        (2, 390, 1), (2, 548, 0), (3, 3, 1), (3, 10, 0), (3, 41, 1), (3, 42, 1),
+                                        (3, 53, 0), (3, 66, 1)])
+@pytest.mark.parametrize("jacobi", [True, False])
+def test_cg_one_launch_matches_the_loop(pf, b200, monkeypatch, dim, N, half, jacobi):
+    """The one-launch CG against the launch-per-step loop, at one, two and four
+    rows per thread, one CTA to all, half and full layouts: FP64 to 1e-10 with
+    the solves' bars (same stop, iterations +-5 %, solution 1e-8); FP32 after 20
+    steps within 5e-4 (20 steps of 6e-8 roundings, a growth of a few hundred);
+    the residual history; stops at the limit, at once and inside."""
+    monkeypatch.setenv("B200LA_HALF_STENCIL", str(half))
+    k = np.exp(np.random.default_rng(N).standard_normal(N ** dim) * 0.5)
+    row, col, val = b200.q1_assemble(dim, N, 0, k)
+    n, bh = len(row) - 1, b200.q1_rhs(N, dim, N)
+    A64 = b200.CSR_lMatrix.from_csr(pf, row, col, val)
+    A32 = A64.CastFrom(b200.F32)
+
+    def solve(A, loop, ctl, x0=0.0):
+        if loop:
+            monkeypatch.setenv("B200LA_GRAPH_LOOP", "1")
+        else:
+            monkeypatch.delenv("B200LA_GRAPH_LOOP", raising=False)
+        cg = b200.CG(pf)
+        cg.SetupOperator(A)
+        cg.SetupPreconditioner(b200.Preconditioner.Jacobi(pf, A) if jacobi else None)
+        cg.InitControl(*ctl)
+        x = pf.vector(np.full(n, x0), A.dtype)
+        return cg.Solve(pf.vector(bh, A.dtype), x, history=200), cg.iter(), cg.history, x.numpy()
+
+    for ctl, x0 in (((20000, 0.0, 1e-10, 1e6), 0.25), ((7, 0.0, 1e-14, 1e6), 0.0), ((0, 0.0, 1e-14, 1e6), 0.5),
+                    ((50, 1e30, 0.0, 1e6), 0.5)):
+        a, c = solve(A64, False, ctl, x0), solve(A64, True, ctl, x0)
+        assert a[0] == c[0] and abs(a[1] - c[1]) <= max(1, c[1] // 20)
+        m = min(len(a[2]), len(c[2]), 30)
+        # (N = 1 has no inner dof: a zero residual, 0 / 0 in both)
+        assert np.allclose(a[2][:m], c[2][:m], rtol=1e-6, atol=1e-12 * c[2][0], equal_nan=True)
+        assert np.array_equal(np.isnan(a[3]), np.isnan(c[3]))
+        assert np.linalg.norm(np.nan_to_num(a[3] - c[3])) <= 1e-8 * np.linalg.norm(np.nan_to_num(c[3]))
+    if half:
+        ctl = (min(20, n // 8), 0.0, 1e-7, 1e12)
+        a, c = solve(A32, False, ctl), solve(A32, True, ctl)
+        assert abs(a[1] - c[1]) <= 1
+        assert np.linalg.norm(np.nan_to_num(a[3] - c[3])) <= 5e-4 * np.linalg.norm(np.nan_to_num(c[3]))
+
+
+def test_cg_one_launch_on_concurrent_contexts(b200):
+    """Two threads with a context each solve at the same time (every launch needs
+    all of its CTAs resident): each gets the result it gets alone."""
+    import threading
+    out = {}
+
+    def work(k):
+        pf = b200.Platform(0)
+        row, col, val = b200.q1_assemble(2, 270 + k)
+        A = b200.CSR_lMatrix.from_csr(pf, row, col, val)
+        cg = b200.CG(pf)
+        cg.SetupOperator(A)
+        cg.SetupPreconditioner(b200.Preconditioner.Jacobi(pf, A))
+        cg.InitControl(300, 0.0, 1e-10, 1e6)
+        b = pf.vector(b200.q1_rhs(3, 2, 270 + k))
+        xs = []
+        for _ in range(8):
+            x = pf.vector(len(row) - 1)
+            cg.Solve(b, x)
+            xs.append(x.numpy())
+        out.setdefault(k, []).append(xs)
+
+    for threads in ([0], [1], [0, 1]):
+        ts = [threading.Thread(target=work, args=(k,)) for k in threads]
+        [t.start() for t in ts]
+        [t.join() for t in ts]
+    for k in (0, 1):
+        alone, together = out[k]
+        assert all(np.array_equal(x, alone[0]) for x in alone + together)
+
+
 def test_captured_graphs_follow_new_objects(pf, b200):
     """A solve after its operator and preconditioner were freed and others made
     (whose handles may get the freed addresses again) runs on the new ones: the
