@@ -52,6 +52,7 @@ struct b200la_ctx {
     b200::DevState *st_host = nullptr;   // pinned mirror
     double *dscal = nullptr;        // device scalars (256)
     double *hscal = nullptr;        // pinned host scalars (256)
+    unsigned hseq = 0;              // number of the last result written straight to hscal
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;     // solver-internal timing
     cudaEvent_t tev0 = nullptr, tev1 = nullptr;   // b200la_timer_start / stop
     void *work = nullptr;           // solver workspace

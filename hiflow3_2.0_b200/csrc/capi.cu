@@ -1123,25 +1123,36 @@ extern "C" int b200la_dot_dev(b200la_ctx *ctx, int dtype, int n, const void *x, 
     return B200LA_OK;
 }
 
+// A dot product whose kernel writes the result, then its number, to page-locked
+// memory that the host polls: no copy behind the kernel and no wait for the
+// stream's completion event.  (lMatrix / lVector programs take two per CG
+// iteration: 2-D 181^2, host-driven CG: 71 -> 43 us an iteration.)  The poll is
+// short; a long kernel, or an error, is left to the stream's own wait.
+static int dot_to_host(b200la_ctx *ctx, int dtype, int n, const void *x, const void *y, bool root, double *result)
+{
+    volatile unsigned *done = reinterpret_cast<volatile unsigned *>(ctx->hscal + 128);
+    volatile double *value = ctx->hscal;
+    const unsigned seq = ++ctx->hseq;
+    CK(launch_dot(ctx_scratch(ctx), dtype, n, x, y, ctx->hscal, root, ctx->stream, done, seq));
+    ctx->launches += 1;
+    bool there = false;
+    for (int i = 0; i < 20000 && !there; ++i) there = *done == seq;
+    std::atomic_thread_fence(std::memory_order_acquire);
+    if (!there) CK(cudaStreamSynchronize(ctx->stream));
+    *result = *value;
+    return B200LA_OK;
+}
+
 extern "C" int b200la_dot(b200la_ctx *ctx, int dtype, int n, const void *x, const void *y, double *result)
 {
-    if (!ctx || !result) return B200LA_ERR_ARG;
-    int rc = b200la_dot_dev(ctx, dtype, n, x, y, ctx->dscal);
-    if (rc) return rc;
-    CK(cudaMemcpyAsync(ctx->hscal, ctx->dscal, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    *result = ctx->hscal[0];
-    return B200LA_OK;
+    if (!ctx || !result || !dt_ok(dtype) || n < 0 || (n && (!x || !y))) return B200LA_ERR_ARG;
+    return dot_to_host(ctx, dtype, n, x, y, false, result);
 }
 
 extern "C" int b200la_nrm2(b200la_ctx *ctx, int dtype, int n, const void *x, double *result)
 {
     if (!ctx || !result || !dt_ok(dtype) || n < 0 || (n && !x)) return B200LA_ERR_ARG;
-    CK(launch_dot(ctx_scratch(ctx), dtype, n, x, x, ctx->dscal, true, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->hscal, ctx->dscal, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    *result = ctx->hscal[0];
-    return B200LA_OK;
+    return dot_to_host(ctx, dtype, n, x, x, true, result);
 }
 
 #define VEC_ARGS_OK (ctx && dt_ok(dtype) && n >= 0)

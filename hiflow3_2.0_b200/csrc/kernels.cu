@@ -44,7 +44,8 @@ inline int stream_grid(const Scratch *s, int n, int per_thread = 4)
 
 template <typename T>
 __global__ void __launch_bounds__(kBlock) dot_kernel(int n, const T *__restrict__ x, const T *__restrict__ y,
-                                                     double *out, bool sqrt_out, const int *gate, Scratch sc)
+                                                     double *out, bool sqrt_out, const int *gate, Scratch sc,
+                                                     volatile unsigned *done, unsigned seq)
 {
     if (gate_closed(gate)) return;
     using V = typename Vec16<T>::type;
@@ -63,7 +64,13 @@ __global__ void __launch_bounds__(kBlock) dot_kernel(int n, const T *__restrict_
     }
     for (int i = nv * W + tid; i < n; i += stride) a += (double)(x[i] * y[i]);
     double v[1] = {a}, o[1];
-    if (grid_reduce<1>(v, sc.partials, sc.ticket, o)) *out = sqrt_out ? sqrt(o[0]) : o[0];
+    if (grid_reduce<1>(v, sc.partials, sc.ticket, o)) {
+        *out = sqrt_out ? sqrt(o[0]) : o[0];
+        if (done) {   // the host polls for its result
+            __threadfence_system();
+            *done = seq;
+        }
+    }
 }
 
 template <typename T>
@@ -301,11 +308,11 @@ __global__ void scale_dev_kernel(int n, const double *coef, bool reciprocal, con
     } while (0)
 
 cudaError_t launch_dot(const Scratch &s, int dtype, int n, const void *x, const void *y, double *out, bool sqrt_out,
-                       cudaStream_t st)
+                       cudaStream_t st, volatile unsigned *done, unsigned seq)
 {
     const int g = stream_grid(&s, n);
     B200_DISPATCH(dtype, dot_kernel<T><<<g, kBlock, 0, st>>>(n, (const T *)x, (const T *)y, out, sqrt_out,
-                                                             nullptr, s));
+                                                             nullptr, s, done, seq));
     return cudaGetLastError();
 }
 
@@ -313,7 +320,8 @@ cudaError_t launch_dot_to(const Scratch &s, int dtype, int n, const void *x, con
                           const int *gate, cudaStream_t st)
 {
     const int g = stream_grid(&s, n);
-    B200_DISPATCH(dtype, dot_kernel<T><<<g, kBlock, 0, st>>>(n, (const T *)x, (const T *)y, out, false, gate, s));
+    B200_DISPATCH(dtype, dot_kernel<T><<<g, kBlock, 0, st>>>(n, (const T *)x, (const T *)y, out, false, gate, s,
+                                                             nullptr, 0u));
     return cudaGetLastError();
 }
 
@@ -321,7 +329,8 @@ cudaError_t launch_dot_norm_to(const Scratch &s, int dtype, int n, const void *x
                                cudaStream_t st)
 {
     const int g = stream_grid(&s, n);
-    B200_DISPATCH(dtype, dot_kernel<T><<<g, kBlock, 0, st>>>(n, (const T *)x, (const T *)x, out, true, gate, s));
+    B200_DISPATCH(dtype, dot_kernel<T><<<g, kBlock, 0, st>>>(n, (const T *)x, (const T *)x, out, true, gate, s,
+                                                             nullptr, 0u));
     return cudaGetLastError();
 }
 

@@ -249,8 +249,9 @@ cudaError_t launch_lattice(const Scratch &s, int dtype, const LatticeDesc &d, co
                            const SpmvOp &op, cudaStream_t st);
 
 // ---- BLAS1 (dtype 0 double, 1 float; scalars in double) ----
+// done (page-locked host memory, optional): set to seq once *out is written.
 cudaError_t launch_dot(const Scratch &s, int dtype, int n, const void *x, const void *y, double *out,
-                       bool sqrt_out, cudaStream_t st);
+                       bool sqrt_out, cudaStream_t st, volatile unsigned *done = nullptr, unsigned seq = 0);
 cudaError_t launch_axpy(int dtype, int n, double a, const void *x, void *y, cudaStream_t st);
 cudaError_t launch_scaleadd(int dtype, int n, double a, const void *x, void *y, cudaStream_t st);
 cudaError_t launch_scale(int dtype, int n, double a, void *y, cudaStream_t st);
