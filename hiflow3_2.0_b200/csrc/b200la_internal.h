@@ -150,8 +150,8 @@ void syncfree_free(b200la_precond *P);
 void graph_cache_clear(b200la_ctx *ctx);
 // cg_fused.cu
 int cg_fused_rows(const b200la_ctx *ctx, const b200la_csr *A);
-cudaError_t cg_fused_run(b200la_ctx *ctx, const b200la_csr *A, const void *invd, const void *b, void *x,
-                         const b200la_control *ctl, double *hist, int hist_len, int rows);
+cudaError_t cg_fused_run(b200la_ctx *ctx, const b200la_csr *A, const void *invd, const void *b, void *x, void *r,
+                         void *p, const b200la_control *ctl, double *hist, int hist_len, int rows);
 // lattice.cu
 namespace lattice {
 bool grid(int n, const int *row, const int *col, int *mx, int *my, int *mz);

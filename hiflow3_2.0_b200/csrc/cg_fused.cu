@@ -17,10 +17,13 @@
 // load (lane b the left one of band b, lane 16 + b the right one).  Values stay
 // in registers where they fit, else they are re-read through L1, which holds
 // up to about 33 MB of them over the GPU.
-//   Bound by the two grid sums and one L2 round trip of the gathers.
+//   Bound by the two grid sums and one L2 round trip of the gathers.  Per
+// iteration, launch per step -> here: 2-D 33^2 15.1 -> 3.3 us, 256^2 16.5 -> 7-8,
+// 512^2 19.8 -> 10; 3-D 41^3 17.2 -> 9, 64^3 23.4 -> 16.6 (FP32 19.3 -> 14).
 #include "b200la.h"
 #include "b200la_internal.h"
 #include "grid_gather.cuh"
+#include "spmv_rows.cuh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -31,6 +34,7 @@ namespace {
 
 constexpr int kCgThreads = 512;
 constexpr int kCgMaxRows = 4;   // rows per thread
+constexpr int kCgStream = -1;   // (instead of a number of rows) the vectors stay in memory
 
 struct CgFusedArgs {
     const void *val;          // st_val, or sh_val (half layout)
@@ -40,6 +44,9 @@ struct CgFusedArgs {
     const void *b, *invd;     // invd null: no preconditioner
     void *x;
     unsigned char *rows;      // a 16-byte word per row
+    // vectors in memory (cg_stream_kernel)
+    void *r, *p;
+    int per_warp, r_shared, l2hint;
     int maxits, hist_len;
     double abstol, reltol, divtol;
     double *hist;
@@ -274,6 +281,155 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_fused_kernel(CgFusedArgs a)
     }
 }
 
+// The same solve for operators beyond the registers: a persistent grid of one
+// 1,024-thread CTA per SM whose warps own every grid-stride chunk of 32 rows.
+// A p (and r, where both fit) stay in shared memory between the phases, so an
+// iteration reads the operator, p, the scaling and x once each beside the gathers,
+// and writes x and p; the CTAs meet in two grid sums and, before p is gathered, a
+// grid barrier.  With a launch per step the same product left 15-23 us an
+// iteration to the two vector kernels, their reduction tails and the gaps between
+// launches.  Per iteration, launch per step -> here: 2-D 600^2 FP64 20.9 -> 14.5
+// us, 1000^2 30.4 -> 20.4; 3-D 70^3 25.4 -> 21.7, 100^3 53.2 -> 46.9 (FP32 36.1 ->
+// 29.0), 128^3 91.9 -> 89.4 (FP32 57.3 -> 52.8).
+constexpr int kStreamThreads = 1024;
+constexpr size_t kStreamSmem = 128 * 1024;   // the rest of the 228 KB is L1 for the gathers
+
+template <typename T, int NB, bool HALF>
+__global__ void __launch_bounds__(kStreamThreads, 1) cg_stream_kernel(CgFusedArgs a)
+{
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    __shared__ typename GridGather<kStreamThreads>::Shared sh;
+    GridGather<kStreamThreads> gg(a.gmem, sh, a.err);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = a.n, last = n - 1, nch = (n + 31) >> 5;
+    const int K = a.per_warp, c0 = blockIdx.x * (kStreamThreads / 32) + warp, cs = gridDim.x * (kStreamThreads / 32);
+    const T *b = static_cast<const T *>(a.b), *invd = static_cast<const T *>(a.invd);
+    T *x = static_cast<T *>(a.x), *p = static_cast<T *>(a.p);
+    T *aps = reinterpret_cast<T *>(s_raw) + tid;                          // A p of the thread's k-th row at 1024 k
+    T *rs = a.r_shared ? aps + (size_t)K * kStreamThreads : nullptr;      // r likewise
+    auto r_at = [&](int k, int r) -> T & { return rs ? rs[(size_t)k * kStreamThreads] : static_cast<T *>(a.r)[r]; };
+    const uint64_t pol = l2_policy(0), pol_v = l2_policy(a.l2hint & 4 ? 1 : 0), pol_own = l2_policy(a.l2hint & 8 ? 1 : 0);
+    int cen[NB];
+#pragma unroll
+    for (int q = 0; q < NB; ++q) cen[q] = a.cen[q];
+    auto product = [&](int c, const T *v) -> T {
+        auto gx = [&](int j) -> T { return v[j]; };
+        if constexpr (HALF)
+            return half_row<NB>(static_cast<const double *>(a.val), a.mask, cen, c, lane, last, pol, pol_own,
+                                (a.l2hint & 16) != 0, gx);
+        else
+            return stencil_row<T, NB>(static_cast<const typename StencilVec<T, stencil_group<T>()>::type *>(a.val), cen, c,
+                                      lane, last, pol_v, gx);
+    };
+    // r = b - A x, p = z = M^-1 r (cg.cc:200-214)
+    double sum[2] = {0.0, 0.0};
+    for (int k = 0, c = c0; c < nch; ++k, c += cs) {
+        const int r = 32 * c + lane;
+        const T s = product(c, x);
+        if (r >= n) continue;
+        const T rv = b[r] - s, z = invd ? rv * invd[r] : rv;
+        r_at(k, r) = rv;
+        p[r] = z;
+        sum[0] += (double)(rv * rv);
+        sum[1] += (double)(rv * z);
+    }
+    gg.template publish<2>(sum);
+    gg.template total<2>(sum);
+    const double res0 = sqrt(sum[0]);
+    auto check = [&](int step, double v) -> int {
+        if (v < a.abstol) return kSuccessAbs;
+        if (v < a.reltol * res0) return kSuccessRel;
+        if (v > a.divtol * res0) return kFailDiv;
+        if (step >= a.maxits) return kFailMaxits;
+        return kIterate;
+    };
+    const bool scribe = blockIdx.x == 0 && tid == 0;
+    int it = 0, status = check(0, res0);
+    double res = res0, rho = sum[1], beta = 0.0, alpha = 0.0;
+    if (scribe && a.hist && a.hist_len > 0) a.hist[0] = res0;
+    while (status == kIterate) {
+        gg.sync();   // p
+        // Ap = A p; alpha = rho / p.Ap (cg.cc:219-220)
+        double pap[1] = {0.0};
+        for (int k = 0, c = c0; c < nch; ++k, c += cs) {
+            const int r = 32 * c + lane;
+            const T s = product(c, p);
+            aps[(size_t)k * kStreamThreads] = s;
+            if (r < n) pap[0] += (double)(p[r] * s);
+        }
+        gg.template publish<1>(pap);
+        gg.template total<1>(pap);
+        alpha = rho / pap[0];
+        const T al = (T)alpha;
+        // r -= alpha Ap; ||r||, r.z (cg.cc:222-240)
+        double v[2] = {0.0, 0.0};
+#pragma unroll 4
+        for (int k = 0; k < K; ++k) {
+            const int r = 32 * (c0 + k * cs) + lane;
+            if (r >= n) continue;
+            const T rv = r_at(k, r) - al * aps[(size_t)k * kStreamThreads], z = invd ? rv * __ldg(invd + r) : rv;
+            r_at(k, r) = rv;
+            v[0] += (double)(rv * rv);
+            v[1] += (double)(rv * z);
+        }
+        gg.template publish<2>(v);
+        // x += alpha p (cg.cc:221) while the sums travel
+#pragma unroll 4
+        for (int k = 0; k < K; ++k) {
+            const int r = 32 * (c0 + k * cs) + lane;
+            if (r < n) x[r] += al * p[r];
+        }
+        gg.template total<2>(v);
+        ++it;
+        res = sqrt(v[0]);
+        status = check(it, res);
+        if (scribe && a.hist && it < a.hist_len) a.hist[it] = res;
+        if (status != kIterate) break;
+        beta = v[1] / rho;
+        rho = v[1];
+        // p = beta p + z (cg.cc:241)
+        const T bt = (T)beta;
+#pragma unroll 4
+        for (int k = 0; k < K; ++k) {
+            const int r = 32 * (c0 + k * cs) + lane;
+            if (r >= n) continue;
+            const T rv = r_at(k, r);
+            p[r] = fma(bt, p[r], invd ? rv * __ldg(invd + r) : rv);
+        }
+    }
+    gg.close();
+    if (scribe) {
+        a.out->iter = it;
+        a.out->status = status;
+        a.out->res = res;
+        a.out->res0 = res0;
+        a.out->rr = res * res;
+        a.out->rho = rho;
+        a.out->beta = beta;
+        a.out->alpha = alpha;
+        a.out->pad0 = (double)*static_cast<volatile int *>(a.err);
+    }
+}
+
+template <typename T, int NB, bool HALF>
+cudaError_t launch_stream(const CgFusedArgs &a, int grid, cudaStream_t st)
+{
+    const size_t sm = (size_t)a.per_warp * kStreamThreads * sizeof(T) * (a.r_shared ? 2 : 1);
+    cudaError_t e = cudaFuncSetAttribute(cg_stream_kernel<T, NB, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)kStreamSmem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = kStreamThreads;
+    cfg.dynamicSmemBytes = sm;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, cg_stream_kernel<T, NB, HALF>, a);
+}
+
 template <typename T, int NB, bool HALF, int E>
 cudaError_t launch(const CgFusedArgs &a, int grid, cudaStream_t st)
 {
@@ -293,6 +449,7 @@ template <typename T, int NB, bool HALF>
 cudaError_t launch_rows(const CgFusedArgs &a, int rows, int grid, cudaStream_t st)
 {
     switch (rows) {
+    case kCgStream: return launch_stream<T, NB, HALF>(a, grid, st);
     case 1: return launch<T, NB, HALF, 1>(a, grid, st);
     case 2: return launch<T, NB, HALF, 2>(a, grid, st);
     default: return launch<T, NB, HALF, 4>(a, grid, st);
@@ -301,8 +458,16 @@ cudaError_t launch_rows(const CgFusedArgs &a, int rows, int grid, cudaStream_t s
 
 }  // namespace
 
-// Rows per thread of the one-launch solve of A, 0 where it does not run: an
-// operator without the stencil layouts, or more rows than the registers hold.
+// chunks per warp of the streaming form
+static size_t stream_per_warp(const b200la_ctx *ctx, int n)
+{
+    const size_t warps = (size_t)std::min(ctx->num_sms, kGatherMaxCtas) * (kStreamThreads / 32);
+    return ((size_t)(n + 31) / 32 + warps - 1) / warps;
+}
+
+// Rows per thread of the one-launch solve of A (or kCgStream), 0 where it does not run: an
+// operator without the stencil layouts, or A p beyond shared memory (2.4 million
+// rows in FP64, 4.8 in FP32).
 // B200LA_CG_FUSED=0 turns it off, and so do the switches that ask for a form
 // of the launch-per-step loop.
 int cg_fused_rows(const b200la_ctx *ctx, const b200la_csr *A)
@@ -312,20 +477,21 @@ int cg_fused_rows(const b200la_ctx *ctx, const b200la_csr *A)
     if (A->n < 1 || A->n != A->m || !A->st_use || (A->st_nb != 3 && A->st_nb != 9)) return 0;
     const bool half = A->sh_use && A->sh_val;
     if (half ? A->dtype != B200LA_F64 : !A->st_val) return 0;
+    const size_t es = A->dtype == B200LA_F64 ? 8 : 4;
     const long long cap = (long long)std::min(ctx->num_sms, kGatherMaxCtas) * kCgThreads;
     for (int rows = 1; rows <= kCgMaxRows; rows *= 2)
         if (A->n <= cap * rows) return rows;
-    return 0;
+    return stream_per_warp(ctx, A->n) * kStreamThreads * es <= kStreamSmem ? kCgStream : 0;
 }
 
 // The whole solve; the final state stands in ctx->st_host once the stream has
 // passed it.  The row words are the context's own and nothing else is written
 // there, so that a word never carries an epoch to come.
-cudaError_t cg_fused_run(b200la_ctx *ctx, const b200la_csr *A, const void *invd, const void *b, void *x,
-                         const b200la_control *ctl, double *hist, int hist_len, int rows)
+cudaError_t cg_fused_run(b200la_ctx *ctx, const b200la_csr *A, const void *invd, const void *b, void *x, void *r,
+                         void *p, const b200la_control *ctl, double *hist, int hist_len, int rows)
 {
     const bool half = A->sh_use && A->sh_val;
-    if (!ctx->rows) {
+    if (rows > 0 && !ctx->rows) {
         const size_t bytes = 16 * (size_t)std::min(ctx->num_sms, kGatherMaxCtas) * kCgThreads * kCgMaxRows;
         cudaError_t e = cudaMalloc(&ctx->rows, bytes);
         if (e == cudaSuccess) e = cudaMemsetAsync(ctx->rows, 0, bytes, ctx->stream);
@@ -349,7 +515,13 @@ cudaError_t cg_fused_run(b200la_ctx *ctx, const b200la_csr *A, const void *invd,
     a.out = ctx->st_host;
     a.gmem = ctx->gather;
     a.err = ctx->dev_err;
-    const int grid = (A->n + kCgThreads * rows - 1) / (kCgThreads * rows);
+    a.r = r;
+    a.p = p;
+    a.per_warp = (int)stream_per_warp(ctx, A->n);
+    a.r_shared = 2 * (size_t)a.per_warp * kStreamThreads * (A->dtype == B200LA_F64 ? 8 : 4) <= kStreamSmem;
+    a.l2hint = A->l2hint;
+    const int grid = rows > 0 ? (A->n + kCgThreads * rows - 1) / (kCgThreads * rows)
+                              : std::min(ctx->num_sms, kGatherMaxCtas);
     ctx->launches += 1;
     if (A->dtype == B200LA_F32)
         return A->st_nb == 3 ? launch_rows<float, 3, false>(a, rows, grid, ctx->stream)

@@ -106,6 +106,22 @@ struct GridGather {
             out[q] = s;
         }
     }
+    // All CTAs meet, and what their threads wrote before may be read after.
+    __device__ void sync()
+    {
+        __syncthreads();
+        ++epoch;
+        if (threadIdx.x == 0) {
+            fence();
+            st_word(word(blockIdx.x, 0), 0.0, epoch);
+        }
+        if ((int)(threadIdx.x & ~31u) < (int)gridDim.x) {
+            if (threadIdx.x < gridDim.x) poll(word(threadIdx.x, 0));
+            __syncwarp();
+            fence();
+        }
+        __syncthreads();
+    }
     // after an unsuccessful poll number i: true when to give up
     __device__ bool stop(long long i)
     {
@@ -119,6 +135,7 @@ struct GridGather {
     }
 
 private:
+    __device__ static void fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
     __device__ double poll(const void *p)
     {
         double v;

@@ -181,7 +181,7 @@ static int cg_core(b200la_ctx *ctx, const b200la_csr *A, const b200la_precond *P
     if (const int rows = pc < 2 ? cg_fused_rows(ctx, A) : 0) {
         DevState *fs = ctx->st_host;
         if (time_it) SK(cudaEventRecord(ctx->ev0, ctx->stream));
-        SK(cg_fused_run(ctx, A, invd, b, x, ctl, hist_dev, hist_len, rows));
+        SK(cg_fused_run(ctx, A, invd, b, x, w.r, w.p, ctl, hist_dev, hist_len, rows));
         if (time_it) SK(cudaEventRecord(ctx->ev1, ctx->stream));
         SK(cudaStreamSynchronize(ctx->stream));
         float ms = 0.f;

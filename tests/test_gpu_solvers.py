@@ -396,11 +396,13 @@ def test_gmres_one_launch_orthogonalisation(pf, b200, n, dtype):
 
 @pytest.mark.parametrize("dim,N,half", [(2, 1, 1), (2, 2, 1), (2, 21, 1), (2, 21, 0), (2, 274, 1), (2, 275, 0), (2, 275, 1),
                                         (2, 390, 1), (2, 548, 0), (3, 3, 1), (3, 10, 0), (3, 41, 1), (3, 42, 1),
-                                        (3, 53, 0), (3, 66, 1)])
+                                        (3, 53, 0), (3, 66, 1), (2, 552, 0), (2, 553, 1), (3, 67, 0),
+                                        (3, 90, 1)])
 @pytest.mark.parametrize("jacobi", [True, False])
 def test_cg_one_launch_matches_the_loop(pf, b200, monkeypatch, dim, N, half, jacobi):
     """The one-launch CG against the launch-per-step loop, at one, two and four
-    rows per thread, one CTA to all, half and full layouts: FP64 to 1e-10 with
+    rows per thread and beyond (vectors in memory; N = 552 is 305,809 rows), one
+    CTA to all, half and full layouts: FP64 to 1e-10 with
     the solves' bars (same stop, iterations +-5 %, solution 1e-8); FP32 after 20
     steps within 5e-4 (20 steps of 6e-8 roundings, a growth of a few hundred);
     the residual history; stops at the limit, at once and inside."""
