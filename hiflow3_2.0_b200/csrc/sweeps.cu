@@ -297,14 +297,15 @@ __global__ void __launch_bounds__(kLevelThreads) level_sweep_cta_kernel(LevelSwe
 // barrier and for remote shared memory.
 //   Measured (one apply, both directions; before: one cp.async look-ahead per
 // thread for rows of up to four entries, a register look-ahead for longer
-// ones): 2-D 512^2 ILU(0), 1,537 levels, FP64 2,470 -> 695 us (0.23 us per
-// level); 256^2 1,060 -> 292 us, FP32 230 us; 150^2 ILU(1) 1,880 -> 390 us.
+// ones): 2-D 512^2 ILU(0), 1,537 levels, FP64 2,470 -> 710 us (0.23 us per
+// level); 256^2 1,060 -> 300 us, FP32 245 us; 150^2 ILU(1) 1,880 -> 410 us.
 constexpr int kPackMaxRows = 512;
 constexpr int pack_rows(int kp) { return kp == 4 ? kPackMaxRows : kp == 8 ? 256 : 192; }   // rows of a tile
 constexpr int kPackMaxStages = 8;
 constexpr int kPackMinStages = 4;
 constexpr int kPackRing = 4096;    // at least kPackMaxStages tiles, so that what lies further back is solved
 constexpr int kPackProducers = 4;   // producer warps
+static_assert(kPackProducers <= kPackMinStages, "two warps must not wait for the same stage's phases at once");
 constexpr int kPackFar = 32;       // far entries of a tile
 constexpr int kPackMaxEntries = 16;
 constexpr size_t kPackSmemCap = 225 * 1024;   // of the 227 KB a CTA can have, less the static part
@@ -385,7 +386,8 @@ struct PackedRow {
 // them in stage `stg`.  A tile may be read from the barrier before the tile
 // ahead of it on (the watching warp has seen it arrive).
 template <typename T, int KP, bool SGS, bool BWD>
-__device__ __forceinline__ void packed_phase(const PackedSweepArgs &a, unsigned char *smem, int cnt, int &stg, int NT)
+__device__ __forceinline__ void packed_phase(const PackedSweepArgs &a, unsigned char *smem, const PackedShared &sh, int cnt,
+                                             int &stg, int NT)
 {
     using Rec = PackRec<T, KP, SGS>;
     constexpr int R = Rec::bytes;
@@ -399,6 +401,9 @@ __device__ __forceinline__ void packed_phase(const PackedSweepArgs &a, unsigned 
     const T *own_at = reinterpret_cast<const T *>(stages + a.own_off) + tid;
     auto next = [&](int s) { return s + 1 == S ? 0 : s + 1; };
     auto header = [&](int s) { return *reinterpret_cast<const int2 *>(stages + s * a.stage_bytes); };
+    // after a wait has run out no tile is read: its bytes may not have arrived
+    // (the flag is read with a header and looked at a level later)
+    auto failed = [&]() { return *static_cast<const volatile int *>(&sh.fail); };
     auto record = [&](PackedRow<T, KP> &q, int s, int2 h) {
         if (tid >= h.y) return;
         const uint4 *p = reinterpret_cast<const uint4 *>(rec_at + s * a.stage_bytes);
@@ -426,7 +431,9 @@ __device__ __forceinline__ void packed_phase(const PackedSweepArgs &a, unsigned 
     };
     int s1 = next(stg), s2 = next(s1);
     packed_barrier(NT + 32);   // the first two tiles are there
+    int fn = failed();
     int2 hc = header(stg), hn = cnt > 1 ? header(s1) : make_int2(0, 0);
+    if (fn) hc.y = 0;
     PackedRow<T, KP> ra, rb;
     record(ra, stg, hc);
     unpack(ra);
@@ -435,6 +442,7 @@ __device__ __forceinline__ void packed_phase(const PackedSweepArgs &a, unsigned 
         T g[KP];
 #pragma unroll
         for (int e = 0; e < KP; ++e) g[e] = active ? *reinterpret_cast<const T *>(smem + cur.at[e]) : T(0);
+        if (fn) hn.y = 0;
         record(nxt, s1, hn);
         T s = T(0);
 #pragma unroll
@@ -452,6 +460,7 @@ __device__ __forceinline__ void packed_phase(const PackedSweepArgs &a, unsigned 
         packed_barrier(NT + 32);
         hc = hn;
         hn = k + 2 < cnt ? header(s2) : make_int2(0, 0);
+        fn = failed();
         s1 = s2;
         s2 = next(s2);
     };
@@ -483,8 +492,8 @@ __global__ void __launch_bounds__(pack_rows(KP) + 32 * (1 + kPackProducers), 1)
     __syncthreads();
     if (tid < NT) {
         int stg = 0;
-        packed_phase<T, KP, SGS, false>(a, s_raw, nf, stg, NT);
-        packed_phase<T, KP, SGS, true>(a, s_raw, nt - nf, stg, NT);
+        packed_phase<T, KP, SGS, false>(a, s_raw, sh, nf, stg, NT);
+        packed_phase<T, KP, SGS, true>(a, s_raw, sh, nt - nf, stg, NT);
         return;
     }
     // bounded waits: after one has run out (reported in *err) nothing waits any more
@@ -560,6 +569,7 @@ __global__ void __launch_bounds__(pack_rows(KP) + 32 * (1 + kPackProducers), 1)
             bulk_g2s(st, a.pack + 16 * (size_t)t.off16, bytes, &sh.full[s], pol);
             if (ob) bulk_g2s(own + q0, vec + q0, ob, &sh.full[s], pol);
         }
+        __syncwarp();   // no lane waits for a later stage while lane 0 has yet to issue this tile
         if (a.nfar) mbar_arrive_cp_async(&sh.full[s]);
         t = t1;
         t1 = t2;
