@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_fused_kernel(CgFusedArgs a)
 // iteration to the two vector kernels, their reduction tails and the gaps between
 // launches.  Per iteration, launch per step -> here: 2-D 600^2 FP64 20.9 -> 14.5
 // us, 1000^2 30.4 -> 20.4; 3-D 70^3 25.4 -> 21.7, 100^3 53.2 -> 46.9 (FP32 36.1 ->
-// 29.0), 128^3 91.9 -> 89.4 (FP32 57.3 -> 52.8).
+// 26.1), 128^3 91.9 -> 89.4 (FP32 57.3 -> 50.7).
 constexpr int kStreamThreads = 1024;
 constexpr size_t kStreamSmem = 128 * 1024;   // the rest of the 228 KB is L1 for the gathers
 
@@ -320,6 +320,18 @@ __global__ void __launch_bounds__(kStreamThreads, 1) cg_stream_kernel(CgFusedArg
             return stencil_row<T, NB>(static_cast<const typename StencilVec<T, stencil_group<T>()>::type *>(a.val), cen, c,
                                       lane, last, pol_v, gx);
     };
+    // The value lines of the warp's first two chunks come into L2 while the CTAs
+    // wait for one another before the product (FP32 100^3 29.0 -> 26.1 us an
+    // iteration, 128^3 52.8 -> 50.7).  Not those of the half layout, whose second
+    // readings they push out of L2 (FP64 128^3 89 -> 97 us).
+    constexpr int kGroup = stencil_group<T>();
+    constexpr int kChunkBytes = 32 * (int)sizeof(T) * kGroup * ((3 * NB + kGroup - 1) / kGroup);
+    auto ahead = [&](int k) {
+        const int c = c0 + k * cs;
+        if (HALF || c >= nch) return;
+        const char *q = static_cast<const char *>(a.val) + (size_t)c * kChunkBytes;
+        for (int o = 128 * lane; o < kChunkBytes; o += 128 * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(q + o));
+    };
     // r = b - A x, p = z = M^-1 r (cg.cc:200-214)
     double sum[2] = {0.0, 0.0};
     for (int k = 0, c = c0; c < nch; ++k, c += cs) {
@@ -347,6 +359,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) cg_stream_kernel(CgFusedArg
     double res = res0, rho = sum[1], beta = 0.0, alpha = 0.0;
     if (scribe && a.hist && a.hist_len > 0) a.hist[0] = res0;
     while (status == kIterate) {
+        ahead(1);
         gg.sync();   // p
         // Ap = A p; alpha = rho / p.Ap (cg.cc:219-220)
         double pap[1] = {0.0};
@@ -378,6 +391,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) cg_stream_kernel(CgFusedArg
             const int r = 32 * (c0 + k * cs) + lane;
             if (r < n) x[r] += al * p[r];
         }
+        ahead(0);
         gg.template total<2>(v);
         ++it;
         res = sqrt(v[0]);
@@ -474,7 +488,7 @@ int cg_fused_rows(const b200la_ctx *ctx, const b200la_csr *A)
 {
     const char *e = std::getenv("B200LA_CG_FUSED");
     if ((e && std::atoi(e) == 0) || std::getenv("B200LA_GRAPH_LOOP") || std::getenv("B200LA_NOGRAPH")) return 0;
-    if (A->n < 1 || A->n != A->m || !A->st_use || (A->st_nb != 3 && A->st_nb != 9)) return 0;
+    if (!ctx->cooperative || A->n < 1 || A->n != A->m || !A->st_use || (A->st_nb != 3 && A->st_nb != 9)) return 0;
     const bool half = A->sh_use && A->sh_val;
     if (half ? A->dtype != B200LA_F64 : !A->st_val) return 0;
     const size_t es = A->dtype == B200LA_F64 ? 8 : 4;

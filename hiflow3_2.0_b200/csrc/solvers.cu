@@ -882,7 +882,7 @@ extern "C" int b200la_gmres(b200la_ctx *ctx, const b200la_csr *A, const b200la_p
     const long long l0 = ctx->launches;
     const size_t ld_el = ldv / es;
     int ev = 0;
-    const int orth = orth_grid(n, es, ctx->num_sms, &ev);
+    const int orth = ctx->cooperative ? orth_grid(n, es, ctx->num_sms, &ev) : 0;
 
     DevState *hs = ctx->st_host;
     state_init(*hs, ctl, nullptr, 0);
