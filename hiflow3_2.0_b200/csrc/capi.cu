@@ -531,6 +531,15 @@ static int build_half(b200la_ctx *ctx, b200la_csr *A)
         return B200LA_OK;
     }
     A->sh_use = 1;
+    // A half layout that about fits L2 (126 MB) streams its own rows evict-first,
+    // so that the solver's vectors stay: an iteration of the FP64 Jacobi-CG, 3-D,
+    // normal -> evict-first: 80^3 (68 MB) 26.5 -> 25.2 us, 90^3 (96 MB) 35.6 -> 31.4,
+    // 100^3 (132 MB) 46.8 -> 44.6, 108^3 (166 MB) 59.1 -> 58.9; larger ones lose
+    // (114^3 66.1 -> 68.5, 128^3 89.0 -> 91.9): their second readings come too late.
+    // Well inside L2 nothing has to be kept from being pushed out (a residual at
+    // 64^3, 35 MB, repeated: 39.5 -> 40.5 us a multigrid level step).
+    if (!std::getenv("B200LA_L2HINT"))
+        A->l2hint = es * len >= 50000000 && es * len <= 150000000 ? A->l2hint | 8 : A->l2hint & ~8;
     // the half layout now carries the operator's products: the full layout's
     // values are dropped (rebuilt from the CSR when the values change)
     if (A->st_use && A->st_val) {
@@ -628,7 +637,7 @@ int csr_upload(b200la_ctx *ctx, int n_rows, int n_cols, int nnz, const int *row,
     // solve 34.8 -> 29.7 ms, MC-SGS apply 138 -> 124 us), and the half
     // layout's three band groups wait on L2, not DRAM, after the first (FP64
     // SpMV 59.6 -> 58.9 us).  The CSR kernels lose with bits 0 and 1 (FP64
-    // CSR CG 71 -> 103 and 88 ms); the half layout gains nothing from bit 3.
+    // CSR CG 71 -> 103 and 88 ms); for bit 3 see build_half.
     A->l2hint = 4 | 16;
     if (const char *h = std::getenv("B200LA_L2HINT")) A->l2hint = std::atoi(h);
     const int cap = spmv_tile_cap(A->cfg);

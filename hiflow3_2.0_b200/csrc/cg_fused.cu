@@ -289,10 +289,11 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_fused_kernel(CgFusedArgs a)
 // grid barrier.  With a launch per step the same product left 15-23 us an
 // iteration to the two vector kernels, their reduction tails and the gaps between
 // launches.  Per iteration, launch per step -> here: 2-D 600^2 FP64 20.9 -> 14.5
-// us, 1000^2 30.4 -> 20.4; 3-D 70^3 25.4 -> 21.7, 100^3 53.2 -> 46.9 (FP32 36.1 ->
+// us, 1000^2 30.4 -> 20.4; 3-D 70^3 25.4 -> 21.7, 100^3 53.2 -> 44.7 (FP32 36.1 ->
 // 26.1), 128^3 91.9 -> 89.4 (FP32 57.3 -> 50.7).
 constexpr int kStreamThreads = 1024;
-constexpr size_t kStreamSmem = 128 * 1024;   // the rest of the 228 KB is L1 for the gathers
+constexpr size_t kStreamSmem = 160 * 1024;   // the rest of the 228 KB is L1 for the gathers
+constexpr size_t kStreamAp = 128 * 1024;     // A p beyond this: launch per step (no gain left at 2.4 million FP64 rows)
 
 template <typename T, int NB, bool HALF>
 __global__ void __launch_bounds__(kStreamThreads, 1) cg_stream_kernel(CgFusedArgs a)
@@ -495,7 +496,7 @@ int cg_fused_rows(const b200la_ctx *ctx, const b200la_csr *A)
     const long long cap = (long long)std::min(ctx->num_sms, kGatherMaxCtas) * kCgThreads;
     for (int rows = 1; rows <= kCgMaxRows; rows *= 2)
         if (A->n <= cap * rows) return rows;
-    return stream_per_warp(ctx, A->n) * kStreamThreads * es <= kStreamSmem ? kCgStream : 0;
+    return stream_per_warp(ctx, A->n) * kStreamThreads * es <= kStreamAp ? kCgStream : 0;
 }
 
 // The whole solve; the final state stands in ctx->st_host once the stream has
