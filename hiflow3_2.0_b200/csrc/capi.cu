@@ -536,8 +536,7 @@ static int build_half(b200la_ctx *ctx, b200la_csr *A)
     // normal -> evict-first: 80^3 (68 MB) 26.5 -> 25.2 us, 90^3 (96 MB) 35.6 -> 31.4,
     // 100^3 (132 MB) 46.8 -> 44.6, 108^3 (166 MB) 59.1 -> 58.9; larger ones lose
     // (114^3 66.1 -> 68.5, 128^3 89.0 -> 91.9): their second readings come too late.
-    // Well inside L2 nothing has to be kept from being pushed out (a residual at
-    // 64^3, 35 MB, repeated: 39.5 -> 40.5 us a multigrid level step).
+    // Well inside L2 (below 50 MB) nothing is pushed out and the normal priority stays.
     if (!std::getenv("B200LA_L2HINT"))
         A->l2hint = es * len >= 50000000 && es * len <= 150000000 ? A->l2hint | 8 : A->l2hint & ~8;
     // the half layout now carries the operator's products: the full layout's

@@ -1,7 +1,7 @@
 // spmv_rows.cuh -- one 32-row chunk of a structured operator times a vector, by
 // one warp, one row per lane: the row sums of the stencil and half stencil
-// layouts (kernels.cuh), shared by the SpMV kernels and the one-launch CG.  gx(j)
-// is the vector's entry j.
+// layouts (kernels.cuh), for the SpMV kernels and the one-launch CG.  gx(j) is the
+// vector's entry j.
 #pragma once
 
 #include "common.cuh"
