@@ -198,6 +198,9 @@ extern "C" int b200la_create(int device, b200la_ctx **out)
         b200la_destroy(ctx);
         return e == cudaErrorMemoryAllocation ? B200LA_ERR_ALLOC : B200LA_ERR_CUDA;
     }
+    // page-locked blocks are handed out again with what their last user left in
+    // them: the completion word of a Dot (dot_to_host) must start below every number
+    std::memset(ctx->hscal, 0, sizeof(double) * 256);
     ctx->stream = ctx->own_stream;
     *out = ctx;
     return B200LA_OK;
@@ -1138,7 +1141,7 @@ extern "C" int b200la_dot_dev(b200la_ctx *ctx, int dtype, int n, const void *x, 
 // short; a long kernel, or an error, is left to the stream's own wait.
 static int dot_to_host(b200la_ctx *ctx, int dtype, int n, const void *x, const void *y, bool root, double *result)
 {
-    volatile unsigned *done = reinterpret_cast<volatile unsigned *>(ctx->hscal + 128);
+    volatile unsigned *done = reinterpret_cast<volatile unsigned *>(ctx->hscal + 128);   // 0 in a new context
     volatile double *value = ctx->hscal;
     const unsigned seq = ++ctx->hseq;
     CK(launch_dot(ctx_scratch(ctx), dtype, n, x, y, ctx->hscal, root, ctx->stream, done, seq));

@@ -320,6 +320,25 @@ def test_blas1_vs_numpy(pf, b200, oracle, n):
                                atol=1e-6 * np.sqrt(n))
 
 
+@pytest.mark.parametrize("op", ["Dot", "Norm2"])
+def test_first_dot_of_a_context_waits_for_its_own_kernel(pf, b200, op):
+    """Contexts made one after another (each gets the page-locked block of the
+    one before, with what its last Dot left there) and after page-locked buffers
+    full of ones were freed: the first Dot / Norm2 is that of its own vectors."""
+    import ctypes as C
+    for k in range(1, 9):
+        if k > 4:
+            held = [pf.host_alloc(2048) for _ in range(64)]
+            for h in held:
+                (C.c_uint32 * 512).from_address(h.value)[:] = [1] * 512
+            for h in held:
+                pf.host_free(h)
+        q = b200.Platform(0)
+        x = q.vector(np.full(1000, float(k)))
+        assert (x.Dot(x) if op == "Dot" else x.Norm2() ** 2) == pytest.approx(1000.0 * k * k, rel=1e-13)
+        q.close()
+
+
 def test_reference_gpu_kernel_baseline(oracle):
     """The reference's own GPU SpMV (kernel_spmv_csr_scalar, built for sm_100a
     into baseline/_ref and timed in bench.py beside the platform's kernels)
