@@ -48,6 +48,7 @@ struct b200la_ctx {
     int *dev_err = nullptr;         // device error flag (bounded waits)
     unsigned char *gather = nullptr;   // words of the cooperative kernels' grid sums (grid_gather.cuh)
     void *rows = nullptr;           // row words of the one-launch CG (made at its first solve)
+    size_t rows_bytes = 0;
     // whether cooperative launches pay: they start when all their CTAs fit at once,
     // which may take long beside a server that keeps every SM busy
     bool cooperative = true;

@@ -163,6 +163,9 @@ int ctx_check_device_error(b200la_ctx *ctx)
     CK(cudaStreamSynchronize(ctx->stream));
     if (h != kDevOk) {
         cudaMemsetAsync(ctx->dev_err, 0, sizeof(int), ctx->stream);
+        // a gather that gave up may leave words of epochs beyond the saved one
+        cudaMemsetAsync(ctx->gather, 0, kGatherBytes, ctx->stream);
+        if (ctx->rows) cudaMemsetAsync(ctx->rows, 0, ctx->rows_bytes, ctx->stream);
         return ctx_msg(ctx, B200LA_ERR_TIMEOUT, "a bounded device wait gave up (error flag " + std::to_string(h) + ")");
     }
     return B200LA_OK;

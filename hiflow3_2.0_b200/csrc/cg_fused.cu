@@ -50,9 +50,10 @@ struct CgFusedArgs {
     int maxits, hist_len;
     double abstol, reltol, divtol;
     double *hist;
-    DevState *out;            // host mirror: the final state
+    DevState *out;            // host mirror: the final state; pad0 set if a wait ran out
     unsigned char *gmem;
     int *err;
+    int first;   // number of a wait's first poll (gather_first)
 };
 
 // The 3 NB values of row 32 c + lane in (band, column) order.
@@ -124,7 +125,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_fused_kernel(CgFusedArgs a)
     constexpr bool kKeep = E * 3 * NB * (int)sizeof(T) <= 144;   // the values stay in registers
     constexpr bool kTrack = E * (NB + 1) * (int)sizeof(T) <= 160;   // and p at the gathered columns
     __shared__ typename GridGather<kCgThreads>::Shared sh;
-    GridGather<kCgThreads> gg(a.gmem, sh, a.err);
+    GridGather<kCgThreads> gg(a.gmem, sh, a.err, a.first);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = a.n, last = n - 1, nch = (n + 31) >> 5;
     const int c0 = (blockIdx.x * (kCgThreads / 32) + warp) * E;   // the warp's chunks
     const T *b = static_cast<const T *>(a.b), *invd = static_cast<const T *>(a.invd);
@@ -147,7 +148,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_fused_kernel(CgFusedArgs a)
     // the words of the columns that chunk c gathers, once they carry `epoch`
     auto gather = [&](int c, T (&w)[NB], T &h) {
         const int r = 32 * c + lane;
-        for (long long i = 0;; ++i) {
+        for (long long i = gg.first;; ++i) {
             bool ready = true;
 #pragma unroll
             for (int q = 0; q <= NB; ++q) {
@@ -263,6 +264,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_fused_kernel(CgFusedArgs a)
         rho = v[1];
     }
     gg.close();
+    if (gg.failed() && threadIdx.x == 0) a.out->pad0 = 1.0;   // by whichever CTA gave up
 #pragma unroll
     for (int e = 0; e < E; ++e) {
         const int r = 32 * (c0 + e) + lane;
@@ -277,7 +279,6 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_fused_kernel(CgFusedArgs a)
         a.out->rho = rho;
         a.out->beta = beta;
         a.out->alpha = alpha;
-        a.out->pad0 = (double)*static_cast<volatile int *>(a.err);
     }
 }
 
@@ -300,7 +301,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) cg_stream_kernel(CgFusedArg
 {
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ typename GridGather<kStreamThreads>::Shared sh;
-    GridGather<kStreamThreads> gg(a.gmem, sh, a.err);
+    GridGather<kStreamThreads> gg(a.gmem, sh, a.err, a.first);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = a.n, last = n - 1, nch = (n + 31) >> 5;
     const int K = a.per_warp, c0 = blockIdx.x * (kStreamThreads / 32) + warp, cs = gridDim.x * (kStreamThreads / 32);
     const T *b = static_cast<const T *>(a.b), *invd = static_cast<const T *>(a.invd);
@@ -412,6 +413,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) cg_stream_kernel(CgFusedArg
         }
     }
     gg.close();
+    if (gg.failed() && threadIdx.x == 0) a.out->pad0 = 1.0;   // by whichever CTA gave up
     if (scribe) {
         a.out->iter = it;
         a.out->status = status;
@@ -421,7 +423,6 @@ __global__ void __launch_bounds__(kStreamThreads, 1) cg_stream_kernel(CgFusedArg
         a.out->rho = rho;
         a.out->beta = beta;
         a.out->alpha = alpha;
-        a.out->pad0 = (double)*static_cast<volatile int *>(a.err);
     }
 }
 
@@ -500,8 +501,8 @@ int cg_fused_rows(const b200la_ctx *ctx, const b200la_csr *A)
 }
 
 // The whole solve; the final state stands in ctx->st_host once the stream has
-// passed it.  The row words are the context's own and nothing else is written
-// there, so that a word never carries an epoch to come.
+// passed it (and counts only if the error flag is clear then).  The row words are
+// the context's own and nothing else is written there.
 cudaError_t cg_fused_run(b200la_ctx *ctx, const b200la_csr *A, const void *invd, const void *b, void *x, void *r,
                          void *p, const b200la_control *ctl, double *hist, int hist_len, int rows)
 {
@@ -511,6 +512,7 @@ cudaError_t cg_fused_run(b200la_ctx *ctx, const b200la_csr *A, const void *invd,
         cudaError_t e = cudaMalloc(&ctx->rows, bytes);
         if (e == cudaSuccess) e = cudaMemsetAsync(ctx->rows, 0, bytes, ctx->stream);
         if (e != cudaSuccess) return e;
+        ctx->rows_bytes = bytes;
     }
     CgFusedArgs a;
     a.val = half ? A->sh_val : A->st_val;
@@ -528,8 +530,10 @@ cudaError_t cg_fused_run(b200la_ctx *ctx, const b200la_csr *A, const void *invd,
     a.hist = hist;
     a.hist_len = hist_len;
     a.out = ctx->st_host;
+    a.out->pad0 = 0.0;
     a.gmem = ctx->gather;
     a.err = ctx->dev_err;
+    a.first = gather_first();
     a.r = r;
     a.p = p;
     a.per_warp = (int)stream_per_warp(ctx, A->n);

@@ -14,8 +14,17 @@
 // Epochs rise through the life of the context.  Words are double-buffered by
 // the epoch's parity: a CTA writes epoch k + 2 only after it has seen k + 1 of
 // every CTA, which each writes after it has read k.  Polls are bounded; after
-// one has run out (reported in the error flag) nothing waits any more.
+// one has run out (reported in the error flag) nothing waits any more, nor in a
+// later launch until the host has seen the flag.  A sum that lacks a word is
+// infinite, which ends a solve by its own stop test.  (A test for it in the CG's
+// loop took 0.1 us of a small iteration's 3.1 and made the streaming form spill:
+// 80^3 FP64 25.1 -> 27.8 us.)  The CTAs' epochs may differ then, so the host clears
+// the words and the saved epoch with the flag (ctx_check_device_error): a word
+// never carries an epoch to come.
 #pragma once
+
+#include <algorithm>
+#include <cstdlib>
 
 #include "common.cuh"
 
@@ -23,8 +32,16 @@ namespace b200 {
 
 constexpr int kGatherMaxQ = 2;         // quantities per sum
 constexpr int kGatherMaxCtas = 160;    // CTAs of a gathering grid
-constexpr long long kGatherSpin = 1LL << 22;
+constexpr long long kGatherSpin = 1LL << 22;   // polls of one wait: several seconds
 constexpr size_t kGatherBytes = 128 * (1 + (size_t)2 * kGatherMaxCtas);   // the last epoch, the words of two epochs
+
+// B200LA_GATHER_SPIN: polls after which a wait gives up (-1: at the first word that is not there yet)
+// -- as the number of the first poll, counted up to kGatherSpin.
+inline int gather_first()
+{
+    const char *e = std::getenv("B200LA_GATHER_SPIN");
+    return e ? (int)(kGatherSpin - std::min(std::max(std::atoll(e), -1LL), kGatherSpin)) : 0;
+}
 
 __device__ __forceinline__ void st_word(void *p, double v, unsigned long long e)
 {
@@ -52,18 +69,26 @@ struct GridGather {
     unsigned long long epoch;
     Shared &sh;
     int *err;
+    const int first;   // number of a wait's first poll
 
     // `mem`: kGatherBytes of the context (the last epoch used, then the words)
-    __device__ GridGather(unsigned char *mem, Shared &s, int *e) : words(mem + 128), sh(s), err(e)
+    __device__ GridGather(unsigned char *mem, Shared &s, int *e, int f)
+        : words(mem + 128), sh(s), err(e), first(f)
     {
         epoch = __ldcg(reinterpret_cast<const unsigned long long *>(mem));
-        if (threadIdx.x == 0) sh.fail = 0;
+        if (threadIdx.x == 0) sh.fail = __ldcg(e) != kDevOk;
         __syncthreads();
     }
     // after the last sum, by CTA 0: the next kernel goes on from there
     __device__ void close()
     {
         if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned long long *>(words - 128) = epoch;
+    }
+    // After the last wait: whether one of this CTA's has run out (or the flag was up before), in all threads.
+    __device__ bool failed()
+    {
+        __syncthreads();
+        return *static_cast<volatile int *>(&sh.fail) != 0;
     }
     // Publish this CTA's sums of v.  (Nothing else is ordered by it: data that
     // CTAs exchange carry epochs themselves, as a fence costs about 1 us.)
@@ -141,7 +166,10 @@ private:
         double v;
         unsigned long long e;
         ld_word(p, v, e);
-        for (long long i = 0; e != epoch && !stop(i); ++i) ld_word(p, v, e);
+        for (long long i = first; e != epoch; ++i) {
+            if (stop(i)) return __longlong_as_double(0x7ff0000000000000LL);
+            ld_word(p, v, e);
+        }
         return v;
     }
     __device__ void *word(int cta, int q)

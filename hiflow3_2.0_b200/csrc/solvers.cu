@@ -650,13 +650,13 @@ constexpr int kOrthThreads = 512;
 template <typename T, int EV>
 __global__ void __launch_bounds__(kOrthThreads) gmres_orth_kernel(int n, int j, int m, const T *__restrict__ w,
                                                                   T *__restrict__ V, size_t ld, GmresDev d,
-                                                                  DevState *st, unsigned char *gmem, int *err)
+                                                                  DevState *st, unsigned char *gmem, int *err, int first_poll)
 {
     if (gate_closed(&st->status)) return;
     using V4 = std::conditional_t<sizeof(T) == 8, double2, float4>;
     constexpr int W = 16 / (int)sizeof(T);
     __shared__ typename GridGather<kOrthThreads>::Shared sh;
-    GridGather<kOrthThreads> gg(gmem, sh, err);
+    GridGather<kOrthThreads> gg(gmem, sh, err, first_poll);
     const int stride = gridDim.x * kOrthThreads, first = blockIdx.x * kOrthThreads + threadIdx.x;
     const bool scribe = blockIdx.x == 0 && threadIdx.x == 0;
     double *Hj = d.H + (size_t)j * (m + 1);
@@ -803,7 +803,9 @@ static cudaError_t launch_gmres_orth(int grid, int ev, int n, int j, int m, cons
     cfg.stream = stream;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    auto go = [&](auto kern) { return cudaLaunchKernelEx(&cfg, kern, n, j, m, (const T *)w, (T *)V, ld, d, st, gmem, err); };
+    auto go = [&](auto kern) {
+        return cudaLaunchKernelEx(&cfg, kern, n, j, m, (const T *)w, (T *)V, ld, d, st, gmem, err, gather_first());
+    };
     switch (ev) {
     case 1: return go(gmres_orth_kernel<T, 1>);
     case 2: return go(gmres_orth_kernel<T, 2>);
@@ -950,14 +952,18 @@ extern "C" int b200la_gmres(b200la_ctx *ctx, const b200la_csr *A, const b200la_p
         int nodes = 0;
         const int kind = P ? P->kind : 0;
         rc = get_graph(ctx, {graph_key(A), graph_key(P), b, x, wk, (const void *)(intptr_t)mb,
-                             (const void *)(intptr_t)(-7 - kind), ctx->stream}, cycle, &exec, &nodes);
+                             (const void *)(intptr_t)(-7 - kind), ctx->stream,
+                             (const void *)(intptr_t)gather_first()}, cycle, &exec, &nodes);
         if (rc) return rc;
         SK(cudaGraphLaunch(exec, ctx->stream));
         graph_launches += nodes;
         SK(cudaMemcpyAsync(hs, ctx->st, sizeof(DevState), cudaMemcpyDeviceToHost, ctx->stream));
         int jend = mb - 1;
         SK(cudaMemcpyAsync(&ctx->hscal[8], d.jend, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        volatile int *flag = reinterpret_cast<volatile int *>(ctx->hscal + 130);
+        SK(cudaMemcpyAsync(const_cast<int *>(flag), ctx->dev_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         SK(cudaStreamSynchronize(ctx->stream));
+        if (*flag != kDevOk) return ctx_check_device_error(ctx);   // a wait has run out: no further cycle
         if (hs->status != kIterate) std::memcpy(&jend, &ctx->hscal[8], sizeof(int));
         // UpdateSolution + preconditioner + x += w   (gmres.cc:404-445)
         gmres_backsub_kernel<<<1, 1, 0, ctx->stream>>>(jend, mb, d);

@@ -472,6 +472,36 @@ def test_cg_one_launch_on_concurrent_contexts(b200):
         assert all(np.array_equal(x, alone[0]) for x in alone + together)
 
 
+@pytest.mark.parametrize("case", ["cg_registers", "cg_memory", "gmres"])
+def test_one_launch_solvers_after_a_wait_that_ran_out(b200, monkeypatch, case):
+    """Waits between the CTAs that give up at once: the solve reports the time-out
+    (whichever CTA met it), and the same solve after it has the bits of the one
+    before -- no word of the failed solve is taken for one of its own."""
+    pf = b200.Platform(0)
+    dim, N = (3, 68) if case == "cg_memory" else (2, 256)
+    row, col, val = b200.q1_assemble(dim, N)
+    A = b200.CSR_lMatrix.from_csr(pf, row, col, val)
+    s = b200.GMRES(pf, 30) if case == "gmres" else b200.CG(pf)
+    s.SetupOperator(A)
+    s.SetupPreconditioner(b200.Preconditioner.Jacobi(pf, A))
+    b = pf.vector(b200.q1_rhs(1, dim, N))
+
+    def solve(maxits):
+        s.InitControl(maxits, 0.0, 1e-12, 1e6)
+        x = pf.vector(len(row) - 1)
+        return s.Solve(b, x), s.iter(), x.numpy()
+
+    want = solve(40)
+    for maxits in (150, 40, 7):
+        monkeypatch.setenv("B200LA_GATHER_SPIN", "-1")
+        with pytest.raises(b200.B200Error) as e:
+            solve(maxits)
+        assert e.value.code == 7
+        monkeypatch.delenv("B200LA_GATHER_SPIN")
+        got = solve(40)
+        assert got[:2] == want[:2] and np.array_equal(got[2], want[2])
+
+
 def test_captured_graphs_follow_new_objects(pf, b200):
     """A solve after its operator and preconditioner were freed and others made
     (whose handles may get the freed addresses again) runs on the new ones: the
