@@ -32,6 +32,21 @@ inline unsigned long long object_uid()
     return next.fetch_add(1, std::memory_order_relaxed);
 }
 
+// Copies and clearings of a set-up: in the order of the context's stream, whose
+// kernels read the buffer next, and done on return.  (The plain calls run on the
+// legacy stream, which a non-blocking stream does not wait for, and may return with
+// the last part of a pageable copy, or all of a device copy or a clearing, to come.)
+inline cudaError_t setup_copy(cudaStream_t s, void *dst, const void *src, size_t bytes)
+{
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, s);
+    return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+}
+inline cudaError_t setup_zero(cudaStream_t s, void *dst, size_t bytes)
+{
+    const cudaError_t e = cudaMemsetAsync(dst, 0, bytes, s);
+    return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+}
+
 struct GraphEntry {
     std::vector<const void *> key;
     cudaGraphExec_t exec = nullptr;

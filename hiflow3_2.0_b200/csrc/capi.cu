@@ -191,12 +191,14 @@ extern "C" int b200la_create(int device, b200la_ctx **out)
     if ((e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking)) ||
         (e = cudaMalloc(&ctx->partials, sizeof(double) * 8 * kMaxGrid)) ||
         (e = cudaMalloc(&ctx->ticket, sizeof(unsigned) * kTicketWords)) || (e = cudaMalloc(&ctx->dev_err, sizeof(int))) ||
-        (e = cudaMalloc(&ctx->gather, kGatherBytes)) || (e = cudaMemset(ctx->gather, 0, kGatherBytes)) ||
+        (e = cudaMalloc(&ctx->gather, kGatherBytes)) || (e = setup_zero(ctx->own_stream, ctx->gather, kGatherBytes)) ||
         (e = cudaMalloc(&ctx->st, sizeof(DevState))) || (e = cudaMalloc(&ctx->dscal, sizeof(double) * 256)) ||
         (e = cudaMallocHost(&ctx->st_host, sizeof(DevState))) ||
         (e = cudaMallocHost(&ctx->hscal, sizeof(double) * 256)) || (e = cudaEventCreate(&ctx->ev0)) ||
-        (e = cudaEventCreate(&ctx->ev1)) || (e = cudaMemset(ctx->ticket, 0, sizeof(unsigned) * kTicketWords)) ||
-        (e = cudaMemset(ctx->dev_err, 0, sizeof(int))) || (e = spmv_configure()) || (e = sweeps_configure())) {
+        (e = cudaEventCreate(&ctx->ev1)) ||
+        (e = setup_zero(ctx->own_stream, ctx->ticket, sizeof(unsigned) * kTicketWords)) ||
+        (e = setup_zero(ctx->own_stream, ctx->dev_err, sizeof(int))) || (e = spmv_configure()) ||
+        (e = sweeps_configure())) {
         ctx->stream = ctx->own_stream;
         b200la_destroy(ctx);
         return e == cudaErrorMemoryAllocation ? B200LA_ERR_ALLOC : B200LA_ERR_CUDA;
@@ -448,7 +450,7 @@ static int build_sell(b200la_ctx *ctx, b200la_csr *A)
         A->sell_len = (size_t)off[nch];
         if ((e = cudaMalloc(&A->sell_off, sizeof(int) * (nch + 1))) ||
             (e = cudaMalloc(&A->sell_val, es * std::max<size_t>(A->sell_len, 32))) ||
-            (e = cudaMemcpy(A->sell_off, off.data(), sizeof(int) * (nch + 1), cudaMemcpyHostToDevice)))
+            (e = setup_copy(ctx->stream, A->sell_off, off.data(), sizeof(int) * (nch + 1))))
             return ctx_fail(ctx, B200LA_ERR_ALLOC, "sliced layout", e);
         A->bytes += sizeof(int) * (nch + 1) + es * A->sell_len;
     }
@@ -582,10 +584,10 @@ static int upload_lines(b200la_ctx *ctx, b200la_csr *A, const std::vector<int> &
     const size_t L = ls.size(), E = std::max<size_t>(el.size(), 1);
     if ((e = cudaMalloc(&A->line_start, sizeof(int) * L)) || (e = cudaMalloc(&A->line_span, sizeof(int) * L)) ||
         (e = cudaMalloc(&A->entry_line, sizeof(int) * E)) || (e = cudaMalloc(&A->entry_lo, sizeof(int) * E)) ||
-        (e = cudaMemcpy(A->line_start, ls.data(), sizeof(int) * L, cudaMemcpyHostToDevice)) ||
-        (e = cudaMemcpy(A->line_span, lsp.data(), sizeof(int) * L, cudaMemcpyHostToDevice)) ||
-        (!el.empty() && (e = cudaMemcpy(A->entry_line, el.data(), sizeof(int) * el.size(), cudaMemcpyHostToDevice))) ||
-        (!el.empty() && (e = cudaMemcpy(A->entry_lo, elo.data(), sizeof(int) * el.size(), cudaMemcpyHostToDevice))))
+        (e = setup_copy(ctx->stream, A->line_start, ls.data(), sizeof(int) * L)) ||
+        (e = setup_copy(ctx->stream, A->line_span, lsp.data(), sizeof(int) * L)) ||
+        (!el.empty() && (e = setup_copy(ctx->stream, A->entry_line, el.data(), sizeof(int) * el.size()))) ||
+        (!el.empty() && (e = setup_copy(ctx->stream, A->entry_lo, elo.data(), sizeof(int) * el.size()))))
         return ctx_fail(ctx, B200LA_ERR_ALLOC, "csr_create: gather lines", e);
     A->nlines = (int)L;
     A->span_sum = 0;
@@ -601,10 +603,10 @@ static int copy_lines(b200la_ctx *ctx, const b200la_csr *A, b200la_csr *B)
     const size_t L = A->nlines, E = std::max(A->ndelta, 1);
     if ((e = cudaMalloc(&B->line_start, sizeof(int) * L)) || (e = cudaMalloc(&B->line_span, sizeof(int) * L)) ||
         (e = cudaMalloc(&B->entry_line, sizeof(int) * E)) || (e = cudaMalloc(&B->entry_lo, sizeof(int) * E)) ||
-        (e = cudaMemcpy(B->line_start, A->line_start, sizeof(int) * L, cudaMemcpyDeviceToDevice)) ||
-        (e = cudaMemcpy(B->line_span, A->line_span, sizeof(int) * L, cudaMemcpyDeviceToDevice)) ||
-        (e = cudaMemcpy(B->entry_line, A->entry_line, sizeof(int) * E, cudaMemcpyDeviceToDevice)) ||
-        (e = cudaMemcpy(B->entry_lo, A->entry_lo, sizeof(int) * E, cudaMemcpyDeviceToDevice)))
+        (e = setup_copy(ctx->stream, B->line_start, A->line_start, sizeof(int) * L)) ||
+        (e = setup_copy(ctx->stream, B->line_span, A->line_span, sizeof(int) * L)) ||
+        (e = setup_copy(ctx->stream, B->entry_line, A->entry_line, sizeof(int) * E)) ||
+        (e = setup_copy(ctx->stream, B->entry_lo, A->entry_lo, sizeof(int) * E)))
         return ctx_fail(ctx, B200LA_ERR_ALLOC, "csr_cast: gather lines", e);
     return B200LA_OK;
 }
@@ -699,10 +701,10 @@ int csr_upload(b200la_ctx *ctx, int n_rows, int n_cols, int nnz, const int *row,
         if ((e = cudaMalloc(&A->pid, sizeof(uint16_t) * n_rows)) ||
             (e = cudaMalloc(&A->pat_off, sizeof(int) * poff.size())) ||
             (e = cudaMalloc(&A->pat_delta, sizeof(int) * std::max<size_t>(pdel.size(), 1))) ||
-            (e = cudaMemcpy(A->pid, pid.data(), sizeof(uint16_t) * n_rows, cudaMemcpyHostToDevice)) ||
-            (e = cudaMemcpy(A->pat_off, poff.data(), sizeof(int) * poff.size(), cudaMemcpyHostToDevice)) ||
+            (e = setup_copy(ctx->stream, A->pid, pid.data(), sizeof(uint16_t) * n_rows)) ||
+            (e = setup_copy(ctx->stream, A->pat_off, poff.data(), sizeof(int) * poff.size())) ||
             (!pdel.empty() &&
-             (e = cudaMemcpy(A->pat_delta, pdel.data(), sizeof(int) * pdel.size(), cudaMemcpyHostToDevice)))) {
+             (e = setup_copy(ctx->stream, A->pat_delta, pdel.data(), sizeof(int) * pdel.size())))) {
             b200la_csr_destroy(A);
             return ctx_fail(ctx, B200LA_ERR_ALLOC, "csr_create: pattern dictionary", e);
         }
@@ -808,10 +810,9 @@ extern "C" int b200la_csr_cast(b200la_ctx *ctx, const b200la_csr *A, int dtype, 
         if ((e = cudaMalloc(&B->pid, sizeof(uint16_t) * A->n)) ||
             (e = cudaMalloc(&B->pat_off, sizeof(int) * (A->npat + 1))) ||
             (e = cudaMalloc(&B->pat_delta, sizeof(int) * std::max(A->ndelta, 1))) ||
-            (e = cudaMemcpy(B->pid, A->pid, sizeof(uint16_t) * A->n, cudaMemcpyDeviceToDevice)) ||
-            (e = cudaMemcpy(B->pat_off, A->pat_off, sizeof(int) * (A->npat + 1), cudaMemcpyDeviceToDevice)) ||
-            (e = cudaMemcpy(B->pat_delta, A->pat_delta, sizeof(int) * std::max(A->ndelta, 1),
-                            cudaMemcpyDeviceToDevice))) {
+            (e = setup_copy(ctx->stream, B->pid, A->pid, sizeof(uint16_t) * A->n)) ||
+            (e = setup_copy(ctx->stream, B->pat_off, A->pat_off, sizeof(int) * (A->npat + 1))) ||
+            (e = setup_copy(ctx->stream, B->pat_delta, A->pat_delta, sizeof(int) * std::max(A->ndelta, 1)))) {
             b200la_csr_destroy(B);
             return ctx_fail(ctx, B200LA_ERR_ALLOC, "csr_cast: pattern dictionary", e);
         }

@@ -463,8 +463,8 @@ extern "C" int b200la_coupled_create(b200la_ctx *ctx, b200la_comm *comm, const b
     if ((e = cudaMalloc(&M->border_idx, sizeof(int) * std::max(n_border, 1))) ||
         (e = cudaMalloc(&M->border, es * std::max(n_border, 1))) ||
         (e = cudaMalloc(&M->ghost, es * std::max(n_ghost, 1))) ||
-        (n_border && (e = cudaMemcpy(M->border_idx, border_indices, sizeof(int) * n_border, cudaMemcpyHostToDevice))) ||
-        (e = cudaMemset(M->ghost, 0, es * std::max(n_ghost, 1))) ||
+        (n_border && (e = setup_copy(ctx->stream, M->border_idx, border_indices, sizeof(int) * n_border))) ||
+        (e = setup_zero(ctx->stream, M->ghost, es * std::max(n_ghost, 1))) ||
         (e = cudaStreamCreateWithFlags(&M->xs, cudaStreamNonBlocking)) ||
         (e = cudaEventCreateWithFlags(&M->packed, cudaEventDisableTiming)) ||
         (e = cudaEventCreateWithFlags(&M->arrived, cudaEventDisableTiming))) {

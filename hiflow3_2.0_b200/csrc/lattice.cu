@@ -471,10 +471,10 @@ int lattice_attach(b200la_ctx *ctx, b200la_csr *A, const b200::host::Csr &Mh, in
     cudaError_t e = cudaMalloc(&dv, es * std::max<size_t>(v.size(), 1));
     if (e != cudaSuccess) return ctx_fail(ctx, B200LA_ERR_ALLOC, "lattice layout", e);
     if (A->dtype == B200LA_F64) {
-        e = cudaMemcpy(dv, v.data(), 8 * v.size(), cudaMemcpyHostToDevice);
+        e = setup_copy(ctx->stream, dv, v.data(), 8 * v.size());
     } else {
         std::vector<float> f(v.begin(), v.end());
-        e = cudaMemcpy(dv, f.data(), 4 * f.size(), cudaMemcpyHostToDevice);
+        e = setup_copy(ctx->stream, dv, f.data(), 4 * f.size());
     }
     if (e != cudaSuccess) {
         cudaFree(dv);

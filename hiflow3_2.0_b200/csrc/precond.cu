@@ -55,10 +55,10 @@ static int upload_vec(b200la_ctx *ctx, const std::vector<double> &v, int dtype, 
     cudaError_t e = cudaMalloc(out, es * std::max<size_t>(n, 1));
     if (e != cudaSuccess) return ctx_fail(ctx, B200LA_ERR_ALLOC, "precond upload", e);
     if (dtype == B200LA_F64) {
-        e = cudaMemcpy(*out, v.data(), 8 * n, cudaMemcpyHostToDevice);
+        e = setup_copy(ctx->stream, *out, v.data(), 8 * n);
     } else {
         std::vector<float> f(v.begin(), v.end());
-        e = cudaMemcpy(*out, f.data(), 4 * n, cudaMemcpyHostToDevice);
+        e = setup_copy(ctx->stream, *out, f.data(), 4 * n);
     }
     if (e != cudaSuccess) return ctx_fail(ctx, B200LA_ERR_CUDA, "precond upload", e);
     return B200LA_OK;
@@ -180,7 +180,7 @@ static int build_block(b200la_ctx *ctx, int kind, int n, const int *row, const i
         return rc;
     }
     cudaError_t e = cudaMalloc(&P->perm_dev, sizeof(int) * n);
-    if (e == cudaSuccess) e = cudaMemcpy(P->perm_dev, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = setup_copy(ctx->stream, P->perm_dev, perm.data(), sizeof(int) * n);
     if (e != cudaSuccess) {
         b200la_precond_destroy(P);
         return ctx_fail(ctx, B200LA_ERR_CUDA, "precond perm", e);

@@ -947,9 +947,9 @@ extern "C" int b200la_serve_start(const b200la_serve_config *cfg, b200la_server 
          cudaMallocHost(&S->h_done, sizeof(int) * ms) == cudaSuccess &&
          cudaMallocHost(&S->h_tiles, sizeof(int) * kTabWords * kLanes) == cudaSuccess &&
          cudaMallocHost(&S->h_admit, sizeof(b200la_server::AdmitStage)) == cudaSuccess;
-    ok = ok && cudaMemset(S->d_done, 0, sizeof(int) * ms) == cudaSuccess &&
-         cudaMemset(S->d_tiles, 0, sizeof(int) * kTabWords * kLanes) == cudaSuccess &&
-         cudaMemset(S->d_sys, 0, sizeof(SysDesc) * ms) == cudaSuccess;
+    ok = ok && setup_zero(S->s_comp, S->d_done, sizeof(int) * ms) == cudaSuccess &&
+         setup_zero(S->s_comp, S->d_tiles, sizeof(int) * kTabWords * kLanes) == cudaSuccess &&
+         setup_zero(S->s_comp, S->d_sys, sizeof(SysDesc) * ms) == cudaSuccess;
     if (!ok) {
         destroy_server(S);
         return B200LA_ERR_ALLOC;

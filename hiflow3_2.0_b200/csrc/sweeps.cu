@@ -761,7 +761,7 @@ static cudaError_t packed_setup(b200la_ctx *ctx, const b200la_precond *P, SyncFr
     if (stages < kPackMinStages) return cudaSuccess;
     cudaError_t e;
     const size_t tb = sizeof(PackTile) * nt;
-    if ((e = cudaMalloc(&plan->ptiles, tb)) || (e = cudaMemcpy(plan->ptiles, tiles.data(), tb, cudaMemcpyHostToDevice)))
+    if ((e = cudaMalloc(&plan->ptiles, tb)) || (e = setup_copy(ctx->stream, plan->ptiles, tiles.data(), tb)))
         return e;
     pack_far_kernel<<<(nt + 3) / 4, 128, 0, ctx->stream>>>(nt, nf, plan->ptiles, P->L->row, P->L->col, P->U->row,
                                                            P->U->col, 0, nullptr);
@@ -775,7 +775,7 @@ static cudaError_t packed_setup(b200la_ctx *ctx, const b200la_precond *P, SyncFr
         t.far0 = (int)nfar;
         nfar += t.nfar;
     }
-    if ((e = cudaMemcpy(plan->ptiles, tiles.data(), tb, cudaMemcpyHostToDevice)) ||
+    if ((e = setup_copy(ctx->stream, plan->ptiles, tiles.data(), tb)) ||
         (e = cudaMalloc(&plan->far, sizeof(int) * std::max<long long>(nfar, 1))) ||
         (e = cudaMalloc(&plan->pack, std::max<size_t>(off, 16))))
         return e;
@@ -846,8 +846,7 @@ int syncfree_setup(b200la_ctx *ctx, b200la_precond *P)
         if (e == cudaSuccess && !plan->kp && cta) {
             plan->nlev = P->nblocks;
             if (!(e = cudaMalloc(&plan->lev_off, sizeof(int) * (P->nblocks + 1))))
-                e = cudaMemcpy(plan->lev_off, P->block_off.data(), sizeof(int) * (P->nblocks + 1),
-                               cudaMemcpyHostToDevice);
+                e = setup_copy(ctx->stream, plan->lev_off, P->block_off.data(), sizeof(int) * (P->nblocks + 1));
         }
         if (e != cudaSuccess) {
             syncfree_free(P);
@@ -879,10 +878,12 @@ int syncfree_setup(b200la_ctx *ctx, b200la_precond *P)
     plan->lg_u = lgU;
     cudaError_t e;
     if ((e = cudaMalloc(&plan->fwd, sizeof(int2) * f.size())) || (e = cudaMalloc(&plan->bwd, sizeof(int2) * bw.size())) ||
-        (e = cudaMemcpy(plan->fwd, f.data(), sizeof(int2) * f.size(), cudaMemcpyHostToDevice)) ||
-        (e = cudaMemcpy(plan->bwd, bw.data(), sizeof(int2) * bw.size(), cudaMemcpyHostToDevice)) ||
-        (e = cudaMalloc(&P->flags, sizeof(unsigned) * P->n)) || (e = cudaMemset(P->flags, 0, sizeof(unsigned) * P->n)) ||
-        (e = cudaMalloc(&P->sync, sizeof(unsigned) * 4)) || (e = cudaMemset(P->sync, 0, sizeof(unsigned) * 4))) {
+        (e = setup_copy(ctx->stream, plan->fwd, f.data(), sizeof(int2) * f.size())) ||
+        (e = setup_copy(ctx->stream, plan->bwd, bw.data(), sizeof(int2) * bw.size())) ||
+        (e = cudaMalloc(&P->flags, sizeof(unsigned) * P->n)) ||
+        (e = setup_zero(ctx->stream, P->flags, sizeof(unsigned) * P->n)) ||
+        (e = cudaMalloc(&P->sync, sizeof(unsigned) * 4)) ||
+        (e = setup_zero(ctx->stream, P->sync, sizeof(unsigned) * 4))) {
         if (plan->fwd) cudaFree(plan->fwd);
         if (plan->bwd) cudaFree(plan->bwd);
         delete plan;

@@ -75,3 +75,21 @@ def test_local_communicators_on_the_host(b200):
         assert L.b200la_comm_destroy(ctypes.c_void_p(arr[q])) == 0
     assert L.b200la_comm_create_local(0, arr) == 1
     assert L.b200la_status_string(13) == b"communicator failed"
+
+
+def test_setup_copies_are_ordered_on_the_context_stream():
+    """The context's stream is non-blocking: it does not wait for copies and
+    clearings on the legacy stream, which plain cudaMemcpy (whose last part of a
+    pageable source may still be under way on return, as may any device-to-device
+    copy) and cudaMemset use.  None of them may fill a buffer that kernels read;
+    copies to the host are done on return."""
+    src = os.path.join(ROOT, "hiflow3_2.0_b200", "csrc")
+    found = []
+    for name in sorted(os.listdir(src)):
+        with open(os.path.join(src, name)) as f:
+            text = f.read()
+        for m in re.finditer(r"\bcuda(Memcpy|Memset)\(", text):
+            call = text[m.start():text.index(";", m.start())].split("||")[0]
+            if "cudaMemcpyDeviceToHost" not in call:
+                found.append((name, call))
+    assert not found, found
