@@ -116,6 +116,7 @@ def lib():
         "b200la_last_error": ([_P], C.c_char_p),
         "b200la_status_string": ([_I], C.c_char_p),
         "b200la_num_sms": ([_P], _I),
+        "b200la_set_cooperative": ([_P, _I], _I),
         "b200la_malloc": ([_P, C.c_size_t, C.POINTER(_P)], _I),
         "b200la_free": ([_P, _P], _I),
         "b200la_memcpy_h2d": ([_P, _P, _P, C.c_size_t], _I),
@@ -474,6 +475,11 @@ class Platform:
 
     def num_sms(self):
         return lib().b200la_num_sms(self.h)
+
+    def set_cooperative(self, on):
+        """Whether the solvers may use cooperative launches (on by default; off
+        for solves that share the device with long-running work)."""
+        self.check(lib().b200la_set_cooperative(self.h, int(on)), "set_cooperative")
 
     def timer_start(self):
         self.check(lib().b200la_timer_start(self.h), "timer_start")

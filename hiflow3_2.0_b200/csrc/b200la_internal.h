@@ -64,8 +64,9 @@ struct b200la_ctx {
     unsigned char *gather = nullptr;   // words of the cooperative kernels' grid sums (grid_gather.cuh)
     void *rows = nullptr;           // row words of the one-launch CG (made at its first solve)
     size_t rows_bytes = 0;
-    // whether cooperative launches pay: they start when all their CTAs fit at once,
-    // which may take long beside a server that keeps every SM busy
+    // Whether solvers use cooperative launches (b200la_set_cooperative).  Such a launch
+    // starts when all its CTAs fit at once and holds its SMs for a whole solve or
+    // Arnoldi step.
     bool cooperative = true;
     b200::DevState *st = nullptr;   // device solver state
     b200::DevState *st_host = nullptr;   // pinned mirror
@@ -81,6 +82,7 @@ struct b200la_ctx {
     long long launches = 0;         // kernels launched through this context
     std::vector<GraphEntry> graphs; // captured solver iteration batches
     std::string msg;
+    cudaError_t last_cuda = cudaSuccess;   // of the last failure
 };
 
 struct b200la_csr {

@@ -32,6 +32,7 @@ int ctx_fail(const b200la_ctx *ctx, int code, const char *what, cudaError_t e)
         char buf[512];
         std::snprintf(buf, sizeof buf, "%s: %s", what, e == cudaSuccess ? "" : cudaGetErrorString(e));
         const_cast<b200la_ctx *>(ctx)->msg = buf;
+        const_cast<b200la_ctx *>(ctx)->last_cuda = e;
     }
     return code;
 }
@@ -247,6 +248,13 @@ extern "C" int b200la_set_stream(b200la_ctx *ctx, void *s)
 }
 
 extern "C" void *b200la_get_stream(b200la_ctx *ctx) { return ctx ? (void *)ctx->stream : nullptr; }
+
+extern "C" int b200la_set_cooperative(b200la_ctx *ctx, int on)
+{
+    if (!ctx) return B200LA_ERR_ARG;
+    ctx->cooperative = on != 0;
+    return B200LA_OK;
+}
 
 extern "C" int b200la_sync(b200la_ctx *ctx)
 {

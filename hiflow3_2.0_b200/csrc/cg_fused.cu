@@ -477,7 +477,7 @@ cudaError_t launch_rows(const CgFusedArgs &a, int rows, int grid, cudaStream_t s
 // chunks per warp of the streaming form
 static size_t stream_per_warp(const b200la_ctx *ctx, int n)
 {
-    const size_t warps = (size_t)std::min(ctx->num_sms, kGatherMaxCtas) * (kStreamThreads / 32);
+    const size_t warps = (size_t)gather_ctas(ctx->num_sms) * (kStreamThreads / 32);
     return ((size_t)(n + 31) / 32 + warps - 1) / warps;
 }
 
@@ -494,23 +494,28 @@ int cg_fused_rows(const b200la_ctx *ctx, const b200la_csr *A)
     const bool half = A->sh_use && A->sh_val;
     if (half ? A->dtype != B200LA_F64 : !A->st_val) return 0;
     const size_t es = A->dtype == B200LA_F64 ? 8 : 4;
-    const long long cap = (long long)std::min(ctx->num_sms, kGatherMaxCtas) * kCgThreads;
+    const long long cap = (long long)gather_ctas(ctx->num_sms) * kCgThreads;
     for (int rows = 1; rows <= kCgMaxRows; rows *= 2)
         if (A->n <= cap * rows) return rows;
     return stream_per_warp(ctx, A->n) * kStreamThreads * es <= kStreamAp ? kCgStream : 0;
 }
 
 // The whole solve; the final state stands in ctx->st_host once the stream has
-// passed it (and counts only if the error flag is clear then).  The row words are
+// passed it (and counts only if the error flag is clear then).  An error means that
+// nothing was launched; cudaErrorCooperativeLaunchTooLarge where the CTAs would not
+// all be resident, cudaErrorMemoryAllocation for want of the row words.  The row words are
 // the context's own and nothing else is written there.
 cudaError_t cg_fused_run(b200la_ctx *ctx, const b200la_csr *A, const void *invd, const void *b, void *x, void *r,
                          void *p, const b200la_control *ctl, double *hist, int hist_len, int rows)
 {
     const bool half = A->sh_use && A->sh_val;
     if (rows > 0 && !ctx->rows) {
-        const size_t bytes = 16 * (size_t)std::min(ctx->num_sms, kGatherMaxCtas) * kCgThreads * kCgMaxRows;
+        const size_t bytes = 16 * (size_t)kGatherMaxCtas * kCgThreads * kCgMaxRows;
         cudaError_t e = cudaMalloc(&ctx->rows, bytes);
-        if (e == cudaSuccess) e = cudaMemsetAsync(ctx->rows, 0, bytes, ctx->stream);
+        if (e == cudaSuccess && (e = cudaMemsetAsync(ctx->rows, 0, bytes, ctx->stream)) != cudaSuccess) {
+            cudaFree(ctx->rows);
+            ctx->rows = nullptr;
+        }
         if (e != cudaSuccess) return e;
         ctx->rows_bytes = bytes;
     }
@@ -540,8 +545,7 @@ cudaError_t cg_fused_run(b200la_ctx *ctx, const b200la_csr *A, const void *invd,
     a.r_shared = 2 * (size_t)a.per_warp * kStreamThreads * (A->dtype == B200LA_F64 ? 8 : 4) <= kStreamSmem;
     a.l2hint = A->l2hint;
     const int grid = rows > 0 ? (A->n + kCgThreads * rows - 1) / (kCgThreads * rows)
-                              : std::min(ctx->num_sms, kGatherMaxCtas);
-    ctx->launches += 1;
+                              : gather_ctas(ctx->num_sms);
     if (A->dtype == B200LA_F32)
         return A->st_nb == 3 ? launch_rows<float, 3, false>(a, rows, grid, ctx->stream)
                              : launch_rows<float, 9, false>(a, rows, grid, ctx->stream);

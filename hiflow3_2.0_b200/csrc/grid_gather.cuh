@@ -35,6 +35,15 @@ constexpr int kGatherMaxCtas = 160;    // CTAs of a gathering grid
 constexpr long long kGatherSpin = 1LL << 22;   // polls of one wait: several seconds
 constexpr size_t kGatherBytes = 128 * (1 + (size_t)2 * kGatherMaxCtas);   // the last epoch, the words of two epochs
 
+// CTAs that a gathering grid may have: one per SM.  (B200LA_GATHER_CTAS: another number.
+// Where they are not all resident at once the launch is refused and the solvers
+// take a launch per step.)
+inline int gather_ctas(int num_sms)
+{
+    const char *e = std::getenv("B200LA_GATHER_CTAS");
+    return std::max(1, std::min(e ? std::atoi(e) : num_sms, kGatherMaxCtas));
+}
+
 // B200LA_GATHER_SPIN: polls after which a wait gives up (-1: at the first word that is not there yet)
 // -- as the number of the first poll, counted up to kGatherSpin.
 inline int gather_first()

@@ -648,7 +648,7 @@ void gmres_loop(b200la_server *S)
     cudaSetDevice(S->device);
     b200la_ctx *ctx = nullptr;
     const bool ok = b200la_create(S->device, &ctx) == B200LA_OK;
-    if (ok) ctx->cooperative = false;   // the batched rounds keep the SMs busy beside it
+    if (ok) b200la_set_cooperative(ctx, 0);   // the batched rounds keep the SMs busy beside it
     for (;;) {
         Req *q = nullptr;
         size_t need = 0;

@@ -178,10 +178,17 @@ static int cg_core(b200la_ctx *ctx, const b200la_csr *A, const b200la_precond *P
     const Scratch sc = ctx_scratch(ctx);
     const long long l0 = ctx->launches;
 
+    bool fused = false;
     if (const int rows = pc < 2 ? cg_fused_rows(ctx, A) : 0) {
-        DevState *fs = ctx->st_host;
         if (time_it) SK(cudaEventRecord(ctx->ev0, ctx->stream));
-        SK(cg_fused_run(ctx, A, invd, b, x, w.r, w.p, ctl, hist_dev, hist_len, rows));
+        const cudaError_t e = cg_fused_run(ctx, A, invd, b, x, w.r, w.p, ctl, hist_dev, hist_len, rows);
+        if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorMemoryAllocation) SK(e);
+        fused = e == cudaSuccess;
+        if (!fused) cudaGetLastError();   // a launch per step needs neither
+    }
+    if (fused) {
+        DevState *fs = ctx->st_host;
+        ctx->launches += 1;
         if (time_it) SK(cudaEventRecord(ctx->ev1, ctx->stream));
         SK(cudaStreamSynchronize(ctx->stream));
         float ms = 0.f;
@@ -781,13 +788,37 @@ __global__ void __launch_bounds__(kOrthThreads) gmres_orth_kernel(int n, int j, 
 static int orth_grid(int n, size_t es, int num_sms, int *ev)
 {
     const long long nv = ((long long)n * (long long)es + 15) / 16;
-    const int cap = std::min(num_sms, kGatherMaxCtas);
+    const int cap = gather_ctas(num_sms);
     for (int e = 1; e <= 8; e *= 2)
         if (nv <= (long long)cap * kOrthThreads * e) {
             *ev = e;
             return (int)std::max(1LL, (nv + (long long)kOrthThreads * e - 1) / ((long long)kOrthThreads * e));
         }
     return 0;
+}
+
+// f(the kernel instance for ev 16-byte vectors per thread)
+template <typename T, class F>
+static auto orth_dispatch(int ev, F f)
+{
+    switch (ev) {
+    case 1: return f(gmres_orth_kernel<T, 1>);
+    case 2: return f(gmres_orth_kernel<T, 2>);
+    case 4: return f(gmres_orth_kernel<T, 4>);
+    default: return f(gmres_orth_kernel<T, 8>);
+    }
+}
+
+// Whether all CTAs of the grid can be on the device at once.  (Asked beforehand:
+// in a captured graph the launch that would say so comes too late.)
+template <typename T>
+static bool orth_resident(const b200la_ctx *ctx, int grid, int ev)
+{
+    int per_sm = 0;
+    const cudaError_t e = orth_dispatch<T>(ev, [&](auto kern) {
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kOrthThreads, 0);
+    });
+    return e == cudaSuccess && grid <= per_sm * ctx->num_sms;
 }
 
 template <typename T>
@@ -803,15 +834,9 @@ static cudaError_t launch_gmres_orth(int grid, int ev, int n, int j, int m, cons
     cfg.stream = stream;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    auto go = [&](auto kern) {
+    return orth_dispatch<T>(ev, [&](auto kern) {
         return cudaLaunchKernelEx(&cfg, kern, n, j, m, (const T *)w, (T *)V, ld, d, st, gmem, err, gather_first());
-    };
-    switch (ev) {
-    case 1: return go(gmres_orth_kernel<T, 1>);
-    case 2: return go(gmres_orth_kernel<T, 2>);
-    case 4: return go(gmres_orth_kernel<T, 4>);
-    default: return go(gmres_orth_kernel<T, 8>);
-    }
+    });
 }
 
 // Back substitution of UpdateSolution (gmres.cc:487-504) into y[0..k].
@@ -884,7 +909,9 @@ extern "C" int b200la_gmres(b200la_ctx *ctx, const b200la_csr *A, const b200la_p
     const long long l0 = ctx->launches;
     const size_t ld_el = ldv / es;
     int ev = 0;
-    const int orth = ctx->cooperative ? orth_grid(n, es, ctx->num_sms, &ev) : 0;
+    int orth = ctx->cooperative ? orth_grid(n, es, ctx->num_sms, &ev) : 0;
+    if (orth && !(dt == B200LA_F64 ? orth_resident<double>(ctx, orth, ev) : orth_resident<float>(ctx, orth, ev)))
+        orth = 0;
 
     DevState *hs = ctx->st_host;
     state_init(*hs, ctl, nullptr, 0);
@@ -951,11 +978,18 @@ extern "C" int b200la_gmres(b200la_ctx *ctx, const b200la_csr *A, const b200la_p
         cudaGraphExec_t exec;
         int nodes = 0;
         const int kind = P ? P->kind : 0;
+        ctx->last_cuda = cudaSuccess;
         rc = get_graph(ctx, {graph_key(A), graph_key(P), b, x, wk, (const void *)(intptr_t)mb,
-                             (const void *)(intptr_t)(-7 - kind), ctx->stream,
+                             (const void *)(intptr_t)(-7 - kind), ctx->stream, (const void *)(intptr_t)orth,
                              (const void *)(intptr_t)gather_first()}, cycle, &exec, &nodes);
+        const cudaError_t le = rc ? ctx->last_cuda : cudaGraphLaunch(exec, ctx->stream);
+        if (orth && le == cudaErrorCooperativeLaunchTooLarge) {   // (a stream limited to some of the SMs)
+            cudaGetLastError();
+            orth = 0;
+            continue;
+        }
         if (rc) return rc;
-        SK(cudaGraphLaunch(exec, ctx->stream));
+        SK(le);
         graph_launches += nodes;
         SK(cudaMemcpyAsync(hs, ctx->st, sizeof(DevState), cudaMemcpyDeviceToHost, ctx->stream));
         int jend = mb - 1;

@@ -85,6 +85,14 @@ int b200la_destroy(b200la_ctx *ctx);
  * or a stream-ordered free on the same stream). */
 int b200la_set_stream(b200la_ctx *ctx, void *cuda_stream);
 void *b200la_get_stream(b200la_ctx *ctx);
+/* Whether b200la_cg, b200la_mpir and b200la_gmres may solve in cooperative launches
+ * (on in a new context).  Such a launch starts once all its thread blocks fit on the
+ * device together and keeps its SMs for a whole CG solve or Arnoldi step: turn it off
+ * (0) for a context whose solves share the device with long-running work that must
+ * not wait for them, or that they would wait for -- a b200la_server, say.  The
+ * solvers then take a launch per step, as they do where the blocks cannot all be
+ * resident. */
+int b200la_set_cooperative(b200la_ctx *ctx, int on);
 /* lVector::Sync (src/linear_algebra/lmp/lvector.h:245) */
 int b200la_sync(b200la_ctx *ctx);
 const char *b200la_last_error(const b200la_ctx *ctx);

@@ -502,6 +502,53 @@ def test_one_launch_solvers_after_a_wait_that_ran_out(b200, monkeypatch, case):
         assert got[:2] == want[:2] and np.array_equal(got[2], want[2])
 
 
+@pytest.mark.parametrize("case", ["cg", "mpir", "gmres"])
+@pytest.mark.parametrize("how", ["switch", "too_large"])
+def test_solvers_without_cooperative_launches(b200, monkeypatch, case, how):
+    """With the context's switch off, and where the grid cannot be resident (160
+    CTAs of which an SM holds one), the solvers take a launch per step and get the
+    same result: the solves' bars of the one-launch tests (steps +-5 %, solution
+    1e-8).  On again, they take one launch (a CG) or one per step (GMRES).  (For
+    GMRES the grid that is too large serves vectors that get launches anyway.)"""
+    pf = b200.Platform(0)
+    if how == "too_large" and pf.num_sms() >= 160:
+        pytest.skip("the device has room for the grid")
+    beyond = case == "gmres" and how == "too_large"
+    N = 106 if beyond else 70                   # 1,225,043 and 357,911 rows
+    row, col, val = b200.q1_assemble(3, N)
+    n = len(row) - 1
+    A = b200.CSR_lMatrix.from_csr(pf, row, col, val)
+    s = {"cg": b200.CG, "mpir": b200.MPIR, "gmres": b200.GMRES}[case](pf)
+    s.SetupOperator(A)
+    if case == "cg":
+        s.SetupPreconditioner(b200.Preconditioner.Jacobi(pf, A))
+    s.InitControl(12 if case == "gmres" else 2000, 0.0, 1e-10, 1e6)
+    b = pf.vector(b200.q1_rhs(1, 3, N))
+
+    def solve():
+        x = pf.vector(n)
+        return s.Solve(b, x), s.iter(), x.numpy(), s.result.launches
+
+    solve()   # (MPIR makes the operator's FP32 scaling in its first solve: two launches)
+    want = solve()
+    for _ in range(2):
+        if how == "switch":
+            pf.set_cooperative(False)
+        else:
+            monkeypatch.setenv("B200LA_GATHER_CTAS", "160")
+        got = solve()
+        assert got[0] == want[0]
+        assert got[3] == want[3] if beyond else got[3] > want[3] + 2 * got[1]
+        assert abs(got[1] - want[1]) <= max(1, want[1] // 20)
+        assert np.linalg.norm(got[2] - want[2]) <= 1e-8 * np.linalg.norm(want[2])
+        if how == "switch":
+            pf.set_cooperative(True)
+        else:
+            monkeypatch.delenv("B200LA_GATHER_CTAS")
+        again = solve()
+        assert again[3] == want[3] and np.array_equal(again[2], want[2])
+
+
 def test_captured_graphs_follow_new_objects(pf, b200):
     """A solve after its operator and preconditioner were freed and others made
     (whose handles may get the freed addresses again) runs on the new ones: the
