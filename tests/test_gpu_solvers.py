@@ -340,6 +340,110 @@ def test_ilu0_level_sweep_beyond_ring(pf, b200, dim, N, kind, monkeypatch):
 
 
 
+def _ls_reference(b200, P, fr, fc, fv, r):
+    """Forward and backward substitution with the host's factors in P's order,
+    the couplings inside a level dropped."""
+    import scipy.sparse as sp
+    import scipy.sparse.linalg as sl
+    n = len(fr) - 1
+    F = sp.csr_matrix((fv, fc, fr), shape=(n, n))[P.perm][:, P.perm].tocoo()
+    level = np.repeat(np.arange(P.nblocks), P.block_sizes)
+    keep = (level[F.row] != level[F.col]) | (F.row == F.col)
+    F = sp.csr_matrix((F.data[keep], (F.row[keep], F.col[keep])), shape=(n, n))
+    L = sp.tril(F, -1, format="csr") + sp.identity(n, format="csr")
+    return sl.spsolve_triangular(sp.triu(F, 0, format="csr"), sl.spsolve_triangular(L, r[P.perm], lower=True),
+                                 lower=False)
+
+
+def _seven_point(N):
+    import scipy.sparse as sp
+    d = sp.diags([-np.ones(N - 1), 2.0 * np.ones(N), -np.ones(N - 1)], [-1, 0, 1])
+    eye = sp.identity(N)
+    A = (sp.kron(sp.kron(d, eye), eye) + sp.kron(sp.kron(eye, d), eye) + sp.kron(sp.kron(eye, eye), d)).tocsr()
+    A.sort_indices()
+    return A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data
+
+
+@pytest.mark.parametrize("what,N", [("q1", 2), ("q1", 33), ("q1", 130), ("7pt", 9), ("7pt", 30), ("7pt", 46)])
+@pytest.mark.parametrize("dtype", [0, 1])
+def test_level_sweep_lookahead(pf, b200, what, N, dtype, monkeypatch):
+    """The sweep with the cp.async look-ahead against substitution with the host's
+    factors: levels of one row to several rows a thread (7-point 46^3: 1,586),
+    rows beyond the ring.  The packed sweep's bars."""
+    row, col, val = b200.q1_assemble(2, N) if what == "q1" else _seven_point(N)
+    r = np.random.default_rng(N).uniform(-1, 1, len(row) - 1)
+    monkeypatch.setenv("B200LA_SYNCFREE", "1")
+    monkeypatch.setenv("B200LA_SWEEP", "lookahead")
+    P = b200.Preconditioner.ILU0(pf, row, col, val, b200.PRECOND_ILU0_LS, dtype)
+    ref = _ls_reference(b200, P, row, col, b200.ilu0(row, col, val), r)
+    z = pf.vector(len(r), dtype)
+    for _ in range(2):
+        P.ApplyPreconditioner(pf.vector(r[P.perm], dtype), z)
+        assert np.max(np.abs(z.numpy() - ref)) <= (2e-5 if dtype else 1e-12) * np.max(np.abs(ref))
+
+
+def test_level_sweep_of_wide_levels_keeps_the_lookahead(pf, b200, monkeypatch):
+    """7-point 70^3: levels of up to 3,675 rows of three entries, whose columns lie
+    beyond the packed stream's ring.  Not slower than with the look-ahead (1,648 us
+    an apply), which the register look-ahead is (1,908)."""
+    row, col, val = _seven_point(70)
+    r = pf.vector(np.random.default_rng(1).uniform(-1, 1, len(row) - 1))
+    us, z = {}, {}
+    for sweep in ("cta", "lookahead", "default"):
+        monkeypatch.delenv("B200LA_SWEEP", raising=False)
+        if sweep != "default":
+            monkeypatch.setenv("B200LA_SWEEP", sweep)
+        P = b200.Preconditioner.ILU0(pf, row, col, val, b200.PRECOND_ILU0_LS)
+        z[sweep] = pf.vector(len(row) - 1)
+        t = []
+        for _ in range(8):
+            pf.timer_start()
+            P.ApplyPreconditioner(r, z[sweep])
+            t.append(pf.timer_stop() * 1e3)
+        us[sweep] = min(t)
+    assert us["default"] <= 1.04 * us["lookahead"] and us["default"] < 0.95 * us["cta"], us
+    for sweep in ("lookahead", "default"):
+        d = np.abs(z[sweep].numpy() - z["cta"].numpy())
+        assert np.max(d) <= 1e-12 * np.max(np.abs(z["cta"].numpy()))
+
+
+@pytest.mark.parametrize("far", [1, 31, 32, 33])
+@pytest.mark.parametrize("near", [1, 6, 12])
+@pytest.mark.parametrize("dtype", [0, 1])
+def test_level_sweep_far_columns(pf, b200, far, near, dtype, monkeypatch):
+    """Levels of 100 rows of which `far` couple 4,500 rows back (beyond the ring of
+    4,096) and, the pattern being symmetric, as many 4,500 rows ahead: far columns of
+    both directions, up to a tile's 32 and past it (another variant then), in rows of
+    4, 8 and 16 entries.  The packed sweep's bars."""
+    import scipy.sparse as sp
+    w, levels = 100, 70
+    n = w * levels
+    rng = np.random.default_rng(100 * far + near)
+    i = np.arange(n)
+    pairs = [(i[w:], i[w:] - w)]                       # the chain that makes the levels
+    k = i[45 * w:]
+    k = k[k % w < far]
+    pairs.append((k, k - 45 * w))
+    for d in range(1, near):
+        k = i[w * (d // 3 + 2):]
+        pairs.append((k, k - w * (d // 3 + 1) - k % w + (k % w + 7 * d) % w))
+    r, c = np.concatenate([p[0] for p in pairs]), np.concatenate([p[1] for p in pairs])
+    A = sp.coo_matrix((rng.uniform(-0.5, 0.5, len(r)), (r, c)), shape=(n, n)).tocsr()
+    A = (A + A.T + sp.identity(n) * 12.0).tocsr()
+    A.sort_indices()
+    row, col, val = A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data
+    monkeypatch.setenv("B200LA_SYNCFREE", "1")
+    monkeypatch.setenv("B200LA_SWEEP", "staged")
+    P = b200.Preconditioner.ILU0(pf, row, col, val, b200.PRECOND_ILU0_LS, dtype)
+    assert P.nblocks == levels and np.array_equal(P.perm, i)
+    x = rng.uniform(-1, 1, n)
+    ref = _ls_reference(b200, P, row, col, b200.ilu0(row, col, val), x)
+    z = pf.vector(n, dtype)
+    for _ in range(2):
+        P.ApplyPreconditioner(pf.vector(x, dtype), z)
+        assert np.max(np.abs(z.numpy() - ref)) <= (2e-5 if dtype else 1e-12) * np.max(np.abs(ref))
+
+
 @pytest.mark.parametrize("n,dtype", [(1, 0), (2, 0), (511, 0), (1025, 1), (4097, 0), (151553, 0), (151553, 1),
                                      (303107, 0), (606211, 1), (640000, 0)])
 def test_gmres_one_launch_orthogonalisation(pf, b200, n, dtype):
