@@ -547,14 +547,20 @@ static int build_half(b200la_ctx *ctx, b200la_csr *A)
         return B200LA_OK;
     }
     A->sh_use = 1;
-    // A half layout that about fits L2 (126 MB) streams its own rows evict-first,
-    // so that the solver's vectors stay: an iteration of the FP64 Jacobi-CG, 3-D,
-    // normal -> evict-first: 80^3 (68 MB) 26.5 -> 25.2 us, 90^3 (96 MB) 35.6 -> 31.4,
-    // 100^3 (132 MB) 46.8 -> 44.6, 108^3 (166 MB) 59.1 -> 58.9; larger ones lose
-    // (114^3 66.1 -> 68.5, 128^3 89.0 -> 91.9): their second readings come too late.
-    // Well inside L2 (below 50 MB) nothing is pushed out and the normal priority stays.
+    // A half layout that about fits L2 (126 MB) streams its own rows evict-first, so
+    // that the vectors stay.  Layout bytes and time, normal -> evict-first, 3-D:
+    //             one-launch CG    product repeated  residual repeated  product, L2 cold  GMRES(30)
+    //   76^3   51 MB                13.2 -> 14.6 us   16.7 -> 17.5 us    22.5 -> 20.5 us   1,609 -> 1,581 us
+    //   80^3   60 MB  28.1 -> 26.0  14.6 -> 14.6      18.7 -> 18.7       22.5 -> 22.5      1,710 -> 1,683
+    //   92^3   90 MB  36.6 -> 30.6  22.8 -> 20.9      28.1 -> 25.1       30.7 -> 30.7      2,548 -> 2,531
+    //  100^3  115 MB  47.2 -> 45.1  28.9 -> 27.8      34.8 -> 33.4       38.1 -> 36.9      2,797 -> 2,810
+    //  104^3  130 MB  52.5 -> 52.5  32.5 -> 31.6      38.1 -> 38.7       41.0 -> 41.0      2,941 -> 2,968
+    //  108^3  145 MB  59.1 -> 58.9  35.0 -> 35.1      41.4 -> 42.3       45.1 -> 44.3      7,380 -> 7,402
+    //  128^3  240 MB  89.0 -> 91.9
+    // (CG: us an iteration, at 90^3 and 105^3 in the rows of 92^3 and 104^3.)  So from 55
+    // to 120 MB; below nothing is pushed out, above the second readings come too late.
     if (!std::getenv("B200LA_L2HINT"))
-        A->l2hint = es * len >= 50000000 && es * len <= 150000000 ? A->l2hint | 8 : A->l2hint & ~8;
+        A->l2hint = es * len >= 55000000 && es * len <= 120000000 ? A->l2hint | 8 : A->l2hint & ~8;
     // the half layout now carries the operator's products: the full layout's
     // values are dropped (rebuilt from the CSR when the values change)
     if (A->st_use && A->st_val) {

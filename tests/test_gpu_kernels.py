@@ -339,6 +339,31 @@ def test_first_dot_of_a_context_waits_for_its_own_kernel(pf, b200, op):
         q.close()
 
 
+def test_half_stencil_l2_rule_does_not_slow_the_product(pf, b200, monkeypatch):
+    """3-D 76^3: a half layout of 51 MB lies well inside L2, where streaming its own
+    rows evict-first takes 14.6 us a repeated product and the normal priority 13.2:
+    the rule keeps the normal one."""
+    row, col, val = b200.q1_assemble(3, 76)
+    x, y = pf.vector(np.ones(len(row) - 1)), pf.vector(len(row) - 1)
+    us = {}
+    for hint in ("20", None):
+        if hint:
+            monkeypatch.setenv("B200LA_L2HINT", hint)
+        else:
+            monkeypatch.delenv("B200LA_L2HINT", raising=False)
+        A = b200.CSR_lMatrix.from_csr(pf, row, col, val)
+        assert A.info()["storage"] == "half-stencil"
+        t = []
+        for _ in range(12):
+            pf.timer_start()
+            for _ in range(40):
+                A.VectorMult(x, y)
+            t.append(pf.timer_stop() * 1e3 / 40)
+        us[hint] = min(t)
+        A.close()
+    assert us[None] <= 1.05 * us["20"], us
+
+
 def test_reference_gpu_kernel_baseline(oracle):
     """The reference's own GPU SpMV (kernel_spmv_csr_scalar, built for sm_100a
     into baseline/_ref and timed in bench.py beside the platform's kernels)
