@@ -572,8 +572,8 @@ __global__ void __launch_bounds__(kBlock, MINB) spmv_half_kernel(CsrView A, Spmv
         const int r0 = c << 5, r = r0 + lane;
         const int he = lane == 0 ? r0 - 1 : r0 + 32;
         if constexpr (sizeof(T) == 8) {
-            // half_row's steps, kept in line: through the function the residual
-            // epilogue spills (64^3: 13.7 -> 14.2 us).
+            // half_row's steps (spmv_rows.cuh), kept in line: through the function the
+            // residual epilogue spills (64^3: 13.7 -> 14.2 us).
             // FP64: groups of three bands, their value loads and gathers
             // issued together (register pressure of one group, not of the row)
             if (A.l2hint & 16) {   // the chunk's own value lines into L2 before the first group's loads
@@ -618,33 +618,33 @@ __global__ void __launch_bounds__(kBlock, MINB) spmv_half_kernel(CsrView A, Spmv
                 }
             }
             if (r < n) epilogue<T, EPI>(r, s, op, acc);
-            continue;
-        }
-        T av[NB][3];
-        HalfRow<T, NB>::values(A.sh_val, cen, c, lane, rows, pol, av);
-        if ((__ldg(mask + c) >> lane) & 1u) {
-            // identity row: its upper slots serve the neighbours; off-diagonals are zero
+        } else {
+            T av[NB][3];
+            HalfRow<T, NB>::values(A.sh_val, cen, c, lane, rows, pol, av);
+            if ((__ldg(mask + c) >> lane) & 1u) {
+                // identity row: its upper slots serve the neighbours; off-diagonals are zero
 #pragma unroll
-            for (int b = 0; b < NB; ++b)
+                for (int b = 0; b < NB; ++b)
 #pragma unroll
-                for (int m = 0; m < 3; ++m)
-                    if (b != U || m != 1) av[b][m] = T(0);
-        }
-        T s = T(0);
+                    for (int m = 0; m < 3; ++m)
+                        if (b != U || m != 1) av[b][m] = T(0);
+            }
+            T s = T(0);
 #pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            const int d = cen[b];
-            const T w = gx(min(max(r + d, 0), last));
-            const T h = edge ? gx(min(max(he + d, 0), last)) : T(0);
-            T left = __shfl_up_sync(0xffffffffu, w, 1);
-            T right = __shfl_down_sync(0xffffffffu, w, 1);
-            if (lane == 0) left = h;
-            if (lane == 31) right = h;
-            s += av[b][0] * left;
-            s += av[b][1] * w;
-            s += av[b][2] * right;
+            for (int b = 0; b < NB; ++b) {
+                const int d = cen[b];
+                const T w = gx(min(max(r + d, 0), last));
+                const T h = edge ? gx(min(max(he + d, 0), last)) : T(0);
+                T left = __shfl_up_sync(0xffffffffu, w, 1);
+                T right = __shfl_down_sync(0xffffffffu, w, 1);
+                if (lane == 0) left = h;
+                if (lane == 31) right = h;
+                s += av[b][0] * left;
+                s += av[b][1] * w;
+                s += av[b][2] * right;
+            }
+            if (r < n) epilogue<T, EPI>(r, s, op, acc);
         }
-        if (r < n) epilogue<T, EPI>(r, s, op, acc);
     }
     if constexpr (reduces<EPI>()) {
         double vv[1] = {acc}, out[1];

@@ -1,7 +1,8 @@
 // spmv_rows.cuh -- one 32-row chunk of a structured operator times a vector, by
-// one warp, one row per lane: the row sums of the stencil and half stencil
-// layouts (kernels.cuh), for the SpMV kernels and the one-launch CG.  gx(j) is the
-// vector's entry j.
+// one warp, one row per lane: the row sums of the stencil layout (kernels.cuh) for the
+// SpMV kernels and the streaming CG, and of the half stencil layout: its values for
+// the SpMV kernels, whose FP64 one keeps half_row's steps in line, and half_row for
+// the streaming CG.  gx(j) is the vector's entry j.
 #pragma once
 
 #include "common.cuh"
@@ -96,28 +97,7 @@ struct HalfRow<double, NB> {
     {
         return q >= 0 ? ld_keep(hv + ((size_t)(q >> 5) * H + p) * 32 + (q & 31), pol) : 0.0;
     }
-    static __device__ __forceinline__ void values(const void *sh, const int (&cen)[NB], int c, int lane, int rows,
-                                                  uint64_t pol, double (&av)[NB][3])
-    {
-        const double *__restrict__ hv = static_cast<const double *>(sh);
-        const int r = (c << 5) + lane;
-        const double *own = hv + (size_t)c * H * 32 + lane;
-        av[U][1] = ld_stream(own, pol);
-        av[U][2] = ld_stream(own + 32, pol);
-#pragma unroll
-        for (int ub = 0; ub < U; ++ub)
-#pragma unroll
-            for (int m = 0; m < 3; ++m) av[U + 1 + ub][m] = ld_stream(own + 32 * (2 + 3 * ub + m), pol);
-        av[U][0] = at(hv, r - 1, 1, pol);
-#pragma unroll
-        for (int b = 0; b < U; ++b) {
-            const int q = r + cen[b], p = 2 + 3 * (U - 1 - b);
-            av[b][0] = at(hv, q - 1, p + 2, pol);
-            av[b][1] = at(hv, q, p + 1, pol);
-            av[b][2] = at(hv, q + 1, p, pol);
-        }
-    }
-    // the three values of band b alone (the same loads as values())
+    // the three values of band b of row 32 c + lane
     static __device__ __forceinline__ void band(const double *__restrict__ hv, int d, int c, int lane, int b,
                                                 uint64_t pol, uint64_t pol_own, double (&a)[3])
     {
@@ -202,7 +182,8 @@ __device__ __forceinline__ T stencil_row(const typename StencilVec<T, stencil_gr
 
 // Half layout, FP64: groups of three bands, their value loads and gathers issued
 // together (register pressure of one group, not of the row); identity rows use
-// their diagonal alone.
+// their diagonal alone.  spmv_half_kernel (spmv.cu) holds the same steps in line and
+// must change with them: a solve's residual is formed by either.
 template <int NB, class GX>
 __device__ __forceinline__ double half_row(const double *__restrict__ hv, const unsigned *__restrict__ mask,
                                            const int (&cen)[NB], int c, int lane, int last, uint64_t pol, uint64_t pol_own,

@@ -545,6 +545,40 @@ def test_cg_one_launch_matches_the_loop(pf, b200, monkeypatch, dim, N, half, jac
         assert np.linalg.norm(np.nan_to_num(a[3] - c[3])) <= 5e-4 * np.linalg.norm(np.nan_to_num(c[3]))
 
 
+@pytest.mark.parametrize("dim,N,dtype,its", [(2, 7, 0, 60), (2, 7, 1, 20), (2, 10, 0, 60), (3, 7, 0, 60), (3, 70, 0, 20),
+                                             (3, 115, 0, 12), (3, 145, 1, 8)])
+def test_cg_one_launch_is_one_launch(pf, b200, monkeypatch, dim, N, dtype, its):
+    """The smallest structured operators (64 rows in 2-D) and those whose r no longer
+    fits shared memory (1,560,896 rows FP64, 3,112,136 FP32) solve in one launch, with
+    the loop's result after as many steps: FP64 1e-10 (a few dozen roundings of 1e-16,
+    a growth of a few hundred), FP32 5e-4.  The first residual is that of the product."""
+    row, col, val = b200.q1_assemble(dim, N)
+    n = len(row) - 1
+    A = b200.CSR_lMatrix.from_csr(pf, row, col, val, dtype=dtype)
+    b = pf.vector(b200.q1_rhs(N, dim, N), dtype)
+    x0 = np.random.default_rng(N).uniform(-1, 1, n)
+    cg = b200.CG(pf)
+    cg.SetupOperator(A)
+    cg.SetupPreconditioner(b200.Preconditioner.Jacobi(pf, A))
+    out = {}
+    for loop in (False, True):
+        if loop:
+            monkeypatch.setenv("B200LA_CG_FUSED", "0")
+        cg.InitControl(min(its, n // 4), 0.0, 1e-10 if dtype == 0 else 1e-6, 1e12)
+        x = pf.vector(x0, dtype)
+        cg.Solve(b, x)
+        assert cg.result.launches > 3 if loop else cg.result.launches == 1
+        out[loop] = x.numpy(), cg.iter()
+        cg.InitControl(0, 0.0, 1e-12, 1e6)
+        x, r = pf.vector(x0, dtype), pf.vector(n, dtype)
+        cg.Solve(b, x)
+        A.Residual(b, x, r)
+        assert cg.result.res0 == pytest.approx(r.Norm2(), rel=1e-5 if dtype else 1e-12)
+    assert abs(out[True][1] - out[False][1]) <= 1
+    d = np.linalg.norm(out[True][0] - out[False][0])
+    assert d <= (5e-4 if dtype else 1e-10) * np.linalg.norm(out[True][0])
+
+
 def test_cg_one_launch_on_concurrent_contexts(b200):
     """Two threads with a context each solve at the same time (every launch needs
     all of its CTAs resident): each gets the result it gets alone."""
