@@ -617,10 +617,10 @@ static int copy_lines(b200la_ctx *ctx, const b200la_csr *A, b200la_csr *B)
     const size_t L = A->nlines, E = std::max(A->ndelta, 1);
     if ((e = cudaMalloc(&B->line_start, sizeof(int) * L)) || (e = cudaMalloc(&B->line_span, sizeof(int) * L)) ||
         (e = cudaMalloc(&B->entry_line, sizeof(int) * E)) || (e = cudaMalloc(&B->entry_lo, sizeof(int) * E)) ||
-        (e = setup_copy(ctx->stream, B->line_start, A->line_start, sizeof(int) * L)) ||
-        (e = setup_copy(ctx->stream, B->line_span, A->line_span, sizeof(int) * L)) ||
-        (e = setup_copy(ctx->stream, B->entry_line, A->entry_line, sizeof(int) * E)) ||
-        (e = setup_copy(ctx->stream, B->entry_lo, A->entry_lo, sizeof(int) * E)))
+        (e = cudaMemcpyAsync(B->line_start, A->line_start, sizeof(int) * L, cudaMemcpyDeviceToDevice, ctx->stream)) ||
+        (e = cudaMemcpyAsync(B->line_span, A->line_span, sizeof(int) * L, cudaMemcpyDeviceToDevice, ctx->stream)) ||
+        (e = cudaMemcpyAsync(B->entry_line, A->entry_line, sizeof(int) * E, cudaMemcpyDeviceToDevice, ctx->stream)) ||
+        (e = cudaMemcpyAsync(B->entry_lo, A->entry_lo, sizeof(int) * E, cudaMemcpyDeviceToDevice, ctx->stream)))
         return ctx_fail(ctx, B200LA_ERR_ALLOC, "csr_cast: gather lines", e);
     return B200LA_OK;
 }
@@ -824,9 +824,11 @@ extern "C" int b200la_csr_cast(b200la_ctx *ctx, const b200la_csr *A, int dtype, 
         if ((e = cudaMalloc(&B->pid, sizeof(uint16_t) * A->n)) ||
             (e = cudaMalloc(&B->pat_off, sizeof(int) * (A->npat + 1))) ||
             (e = cudaMalloc(&B->pat_delta, sizeof(int) * std::max(A->ndelta, 1))) ||
-            (e = setup_copy(ctx->stream, B->pid, A->pid, sizeof(uint16_t) * A->n)) ||
-            (e = setup_copy(ctx->stream, B->pat_off, A->pat_off, sizeof(int) * (A->npat + 1))) ||
-            (e = setup_copy(ctx->stream, B->pat_delta, A->pat_delta, sizeof(int) * std::max(A->ndelta, 1)))) {
+            (e = cudaMemcpyAsync(B->pid, A->pid, sizeof(uint16_t) * A->n, cudaMemcpyDeviceToDevice, ctx->stream)) ||
+            (e = cudaMemcpyAsync(B->pat_off, A->pat_off, sizeof(int) * (A->npat + 1), cudaMemcpyDeviceToDevice,
+                                 ctx->stream)) ||
+            (e = cudaMemcpyAsync(B->pat_delta, A->pat_delta, sizeof(int) * std::max(A->ndelta, 1),
+                                 cudaMemcpyDeviceToDevice, ctx->stream))) {
             b200la_csr_destroy(B);
             return ctx_fail(ctx, B200LA_ERR_ALLOC, "csr_cast: pattern dictionary", e);
         }
