@@ -18,8 +18,9 @@
 // in registers where they fit, else they are re-read through L1, which holds
 // up to about 33 MB of them over the GPU.
 //   Bound by the two grid sums and one L2 round trip of the gathers.  Per
-// iteration, launch per step -> here: 2-D 33^2 15.1 -> 3.3 us, 256^2 16.5 -> 7-8,
-// 512^2 19.8 -> 10; 3-D 41^3 17.2 -> 9, 64^3 23.4 -> 16.6 (FP32 19.3 -> 14).
+// iteration, launch per step -> here: 2-D 33^2 15.1 -> 3.4 us (up to 7 on a box that
+// spreads its three CTAs), 256^2 16.5 -> 7-8, 512^2 19.8 -> 11; 3-D 41^3 17.2 -> 9.7,
+// 64^3 23.4 -> 16.7 (FP32 19.3 -> 14.5).
 #include "b200la.h"
 #include "b200la_internal.h"
 #include "grid_gather.cuh"
@@ -289,9 +290,9 @@ __global__ void __launch_bounds__(kCgThreads, 1) cg_fused_kernel(CgFusedArgs a)
 // and writes x and p; the CTAs meet in two grid sums and, before p is gathered, a
 // grid barrier.  With a launch per step the same product left 15-23 us an
 // iteration to the two vector kernels, their reduction tails and the gaps between
-// launches.  Per iteration, launch per step -> here: 2-D 600^2 FP64 20.9 -> 14.5
-// us, 1000^2 30.4 -> 20.4; 3-D 70^3 25.4 -> 21.7, 100^3 53.2 -> 44.7 (FP32 36.1 ->
-// 26.1), 128^3 91.9 -> 89.4 (FP32 57.3 -> 50.7).
+// launches.  Per iteration, launch per step -> here, in one call: 2-D 600^2 FP64
+// 20.2 -> 13.8 us, 1000^2 29.4 -> 20.4; 3-D 70^3 25.2 -> 21.2, 100^3 50.5 -> 44.6 (FP32
+// 35.4 -> 25.9), 108^3 59.1 -> 57.7, 128^3 88.5 -> 88.7 (FP32 57.2 -> 50.5).
 constexpr int kStreamThreads = 1024;
 constexpr size_t kStreamSmem = 160 * 1024;   // the rest of the 228 KB is L1 for the gathers
 constexpr size_t kStreamAp = 128 * 1024;     // A p beyond this: launch per step (no gain left at 2.4 million FP64 rows)
@@ -324,7 +325,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) cg_stream_kernel(CgFusedArg
     };
     // The value lines of the warp's first two chunks come into L2 while the CTAs
     // wait for one another before the product (FP32 100^3 29.0 -> 26.1 us an
-    // iteration, 128^3 52.8 -> 50.7).  Not those of the half layout, whose second
+    // iteration, 128^3 52.8 -> 50.7, in one call).  Not those of the half layout, whose second
     // readings they push out of L2 (FP64 128^3 89 -> 97 us).
     constexpr int kGroup = stencil_group<T>();
     constexpr int kChunkBytes = 32 * (int)sizeof(T) * kGroup * ((3 * NB + kGroup - 1) / kGroup);
