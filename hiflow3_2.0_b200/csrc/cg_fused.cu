@@ -18,7 +18,7 @@
 // in registers where they fit, else they are re-read through L1, which holds
 // up to about 33 MB of them over the GPU.
 //   Bound by the two grid sums and one L2 round trip of the gathers.  Per
-// iteration, launch per step -> here: 2-D 33^2 15.1 -> 3.4 us (up to 7 on a box that
+// iteration, launch per step -> here: 2-D 33^2 15.1 -> 3.4 us (up to 7 where the device
 // spreads its three CTAs), 256^2 16.5 -> 7-8, 512^2 19.8 -> 11; 3-D 41^3 17.2 -> 9.7,
 // 64^3 23.4 -> 16.7 (FP32 19.3 -> 14.5).
 #include "b200la.h"
